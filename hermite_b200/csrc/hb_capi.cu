@@ -224,7 +224,46 @@ const TuneEntry *lookup_tuning(int order, bool mixed, int n, int nact)
     return best;
 }
 
-// Launch shape for the force kernel: the tuned variant and j-slice count of
+// The automatic launch shape: CTAs of two warps, 64 i-particles (shape 8), or
+// 32 with the two warps splitting every j tile (shape 11), and many j-slices.
+//
+// What bounds the choice: a grid that just exceeds a whole number of waves
+// runs one wave more for a few CTAs (6th order, N = 262144, nact = 3001 in the
+// shape and slice count measured for 2^12: 3540 us), and CTAs that start
+// together do not end together, so a single wave leaves SMs part empty.  Small
+// CTAs in several waves fill both gaps: 2691 us at 8 waves, 290-296 Gint/s
+// at any nact from 500 up, 84 % of the FP64 pipe.  That takes more slices than
+// the last CTA of an i-tile could add alone, hence launch_reduce.
+//
+// Shape 11 halves the padding of nact to whole i-tiles and the chunks a warp
+// takes in turn; it wins up to 64 particles and where all pairs together are
+// few (N = 32768, 6th order, nact = 300: 48.6 against 51.3 us; N = 262144,
+// nact = 500: 493 against 480 us).
+constexpr int kShapeWide = 8, kShapeNarrow = 11;
+constexpr long long kNarrowUnits = 12288;      // 64-particle tiles x chunks
+
+int auto_variant(const hb_ctx *c, int nact)
+{
+    const long long units = (long long)((nact + 63) / 64) * (c->npad / 32);
+    return nact <= 64 || units <= kNarrowUnits ? kShapeNarrow : kShapeWide;
+}
+
+// j-slices of the automatic shape; `resident` CTAs of it run at once.
+int auto_slices(int v, int gx, int nchunk, int resident)
+{
+    const double x = (double)gx * nchunk / resident;       // chunks per resident CTA
+    // Large steps: 8 waves, slices of at least 8 chunks.  Small ones (the
+    // narrow shape): a CTA takes about 0.7 us per chunk in turn, and the reduce
+    // grows with the slices, past 256 of them most; the rule is within 2 us of
+    // the best of c = 1, 2, 4, 8 over 4th to 8th order, N = 1024 ... 262144.
+    double c = 8.0;
+    if (v == kShapeNarrow) c = std::max(1.0, std::min(8.0, std::max(2.0 * std::sqrt(x), nchunk / 256.0)));
+    c = std::max(c, x / 8.0);
+    return std::max(1, (int)(nchunk / c));
+}
+
+// Launch shape for a given slice count (hb_set_force_shape with an automatic
+// shape): the tuned variant and j-slice count of
 // the nearest bucket (the slice count rescaled to keep the measured number
 // of CTAs), else a heuristic; then the slice count is clamped so that each
 // CTA keeps at least 8 chunks and the partials fit in the scratch buffer.
@@ -276,8 +315,9 @@ int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
         ctx->launches++;
         return HB_OK;
     }
+    const bool automatic = ctx->variant_override < 0 && ctx->jsplit_override == 0;
     int jsplit_hint = 0;
-    const int v = pick_variant(ctx, nact, &jsplit_hint);
+    const int v = automatic ? auto_variant(ctx, nact) : pick_variant(ctx, nact, &jsplit_hint);
     const ForceVariant *fv = force_variant(ctx->order, mixed, v);
     if (!fv) return fail(ctx, HB_ERR_INVALID, "force variant %d does not exist", v);
     const int m = mixed ? 1 : 0;
@@ -291,14 +331,19 @@ int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
     }
     const int nchunk = ctx->npad / 32;
     const int gx = (nact + fv->ti - 1) / fv->ti;
-    int S = ctx->jsplit_override > 0 ? ctx->jsplit_override : jsplit_hint;
-    if (S <= 0) {
-        const int target = ctx->nsm * ctx->blocks_per_sm[m][v];
-        S = gx >= target ? 1 : (target + gx - 1) / gx;
-        // at least 8 chunks (256 j) per CTA and 2 chunks per j-warp
-        S = std::min(S, std::max(1, nchunk / std::max(8, 2 * fv->wj)));
+    int S;
+    if (automatic) {
+        S = auto_slices(v, gx, nchunk, ctx->nsm * ctx->blocks_per_sm[m][v]);
+    } else {
+        S = ctx->jsplit_override > 0 ? ctx->jsplit_override : jsplit_hint;
+        if (S <= 0) {
+            const int target = ctx->nsm * ctx->blocks_per_sm[m][v];
+            S = gx >= target ? 1 : (target + gx - 1) / gx;
+            // at least 8 chunks (256 j) per CTA and 2 chunks per j-warp
+            S = std::min(S, std::max(1, nchunk / std::max(8, 2 * fv->wj)));
+        }
+        S = std::max(1, std::min(S, ctx->jsplit_override > 0 ? nchunk : std::max(1, nchunk / 8)));
     }
-    S = std::max(1, std::min(S, ctx->jsplit_override > 0 ? nchunk : std::max(1, nchunk / 8)));
     if (S > 1) {
         const size_t need_per_slice = (size_t)gx * fv->ti * ctx->F;
         const size_t smax = ctx->partial_cap / need_per_slice;
@@ -324,6 +369,19 @@ int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
     a.counter = ctx->d_counter;
     a.err = ctx->d_err;
     a.spin = ctx->wait_limit;
+    if (automatic) {
+        // the predictor pass, the force and the sum of the slices, chained by
+        // programmatic dependent launch
+        a.deferred = 1;
+        HB_CK(launch_pdl(fv->kern, dim3(gx, S), threads, fv->smem, ctx->stream, a));
+        ctx->launches++;
+        if (S > 1) {
+            HB_CK(launch_reduce(ctx->d_partial, (size_t)gx * fv->ti * ctx->F, S, nact * ctx->F,
+                                force_out_dev, ctx->stream));
+            ctx->launches++;
+        }
+        return HB_OK;
+    }
     fv->kern<<<dim3(gx, S), threads, fv->smem, ctx->stream>>>(a);
     HB_CK(cudaGetLastError());
     ctx->launches++;

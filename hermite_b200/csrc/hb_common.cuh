@@ -125,6 +125,16 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
     return false;
 }
 
+// Programmatic dependent launch: let the next kernel of the stream be scheduled
+// now, then wait until the previous kernel's results are visible.  (Between
+// kernels launched with programmatic stream serialisation; otherwise both
+// instructions are no-ops.)
+__device__ __forceinline__ void pdl_enter()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ void raise_error(int *err, int code)
 {
     if (err) atomicCAS(err, kErrNone, code);

@@ -341,7 +341,8 @@ __device__ __forceinline__ void force_epilogue(double (&f)[NI][Frc<ORDER>::words
         return;
     }
 
-    // j-split across CTAs: publish this slice's partial, last CTA reduces.
+    // j-split across CTAs: publish this slice's partial; a reduce launch adds
+    // the slices (a.deferred), or the last CTA of the i-tile does.
     const size_t ispan = (size_t)gridDim.x * TI;
     if (jg == 0) {
 #pragma unroll
@@ -351,6 +352,7 @@ __device__ __forceinline__ void force_epilogue(double (&f)[NI][Frc<ORDER>::words
             for (int c = 0; c < F; ++c) a.partial[((size_t)sl * ispan + i) * F + c] = f[n][c];
         }
     }
+    if (a.deferred) return;
     __threadfence();
     __syncthreads();
     if (tid == 0) s_last = (atomicAdd(&a.counter[blockIdx.x], 1u) == (unsigned)(S - 1));
@@ -417,6 +419,7 @@ force_kernel(ForceArgs a)
     unsigned char *ptile = smem + Sh::ring_bytes;          // fused only
     constexpr int RB = Rec<ORDER>::bytes;
 
+    pdl_enter();   // the predictor pass, where it is chained to this launch
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ig = warp % WI, jg = warp / WI;
     const int S = gridDim.y, sl = blockIdx.y;

@@ -43,16 +43,6 @@ constexpr int kBigNact = HB_BIG_NACT;
 #define HB_ITEMS_TARGET_PCT 100
 #endif
 
-// Programmatic dependent launch: let the next kernel of the step be
-// scheduled now, then wait until the previous kernel's results are visible.
-// (The step's kernels are launched with programmatic stream serialisation;
-// without it both instructions are no-ops.)
-__device__ __forceinline__ void pdl_enter()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // ---------------------------------------------------------------------------
 template <int ORDER>
 __device__ __forceinline__ void min_phase(const double *__restrict__ jp, const double *__restrict__ dt,
@@ -777,31 +767,14 @@ __global__ void energy_final_kernel(const double *part, int nblk, double *out)
 
 constexpr int kEnergyBlocks = 256;
 
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*kern)(KArgs...), int grid, int block, int smem, cudaStream_t s,
-                              Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 template <int ORDER>
 static cudaError_t launch_step(const IntegratorLaunch &L, cudaStream_t s)
 {
     const int nb = std::min((L.n + 255) / 256, L.nsm * 8);
-    cudaError_t e = launch_pdl(sched_min_kernel<ORDER>, nb, 256, 0, s, (const double *)L.jp,
+    cudaError_t e = launch_pdl(sched_min_kernel<ORDER>, dim3(nb), 256, 0, s, (const double *)L.jp,
                                (const double *)L.dt, L.n, L.sched);
     if (e == cudaSuccess)
-        e = launch_pdl(sched_compact_kernel<ORDER>, nb, 256, 0, s, (const double *)L.jp,
+        e = launch_pdl(sched_compact_kernel<ORDER>, dim3(nb), 256, 0, s, (const double *)L.jp,
                        (const double *)L.dt, L.n, L.sched, L.ilist);
     ItemsArgs a{L.jp, L.ilist, L.sched, L.force, L.partial, L.counter, L.err, L.n, L.nchunk,
                 L.partial_cap, L.target_items, kBigNact};
@@ -809,28 +782,28 @@ static cudaError_t launch_step(const IntegratorLaunch &L, cudaStream_t s)
     // nact (known on the device only) returns at once
     if constexpr (ORDER == 9) {   // double-double positions: FP64 only
         if (e == cudaSuccess)
-            e = launch_pdl(force_items_kernel<ORDER, false>, L.items_grid, 128, L.smem_fp64, s, a);
+            e = launch_pdl(force_items_kernel<ORDER, false>, dim3(L.items_grid), 128, L.smem_fp64, s, a);
         if (e == cudaSuccess)
-            e = launch_pdl(force_items_big_kernel<ORDER, false>, L.big_grid, 128,
+            e = launch_pdl(force_items_big_kernel<ORDER, false>, dim3(L.big_grid), 128,
                            BigShape<ORDER, false>::smem_bytes, s, a);
     } else {
         if (e == cudaSuccess) {
             if (L.mixed)
-                e = launch_pdl(force_items_kernel<ORDER, true>, L.items_grid, 128, L.smem_mixed, s, a);
+                e = launch_pdl(force_items_kernel<ORDER, true>, dim3(L.items_grid), 128, L.smem_mixed, s, a);
             else
-                e = launch_pdl(force_items_kernel<ORDER, false>, L.items_grid, 128, L.smem_fp64, s, a);
+                e = launch_pdl(force_items_kernel<ORDER, false>, dim3(L.items_grid), 128, L.smem_fp64, s, a);
         }
         if (e == cudaSuccess) {
             if (L.mixed)
-                e = launch_pdl(force_items_big_kernel<ORDER, true>, L.big_grid, 128,
+                e = launch_pdl(force_items_big_kernel<ORDER, true>, dim3(L.big_grid), 128,
                                BigShape<ORDER, true>::smem_bytes, s, a);
             else
-                e = launch_pdl(force_items_big_kernel<ORDER, false>, L.big_grid, 128,
+                e = launch_pdl(force_items_big_kernel<ORDER, false>, dim3(L.big_grid), 128,
                                BigShape<ORDER, false>::smem_bytes, s, a);
         }
     }
     if (e == cudaSuccess)
-        e = launch_pdl(correct_kernel<ORDER>, std::max(1, std::min(nb, L.nsm * 4)), 256, 0, s, L.jp,
+        e = launch_pdl(correct_kernel<ORDER>, dim3(std::max(1, std::min(nb, L.nsm * 4))), 256, 0, s, L.jp,
                        L.dt, (const double *)L.force, (const int *)L.ilist, L.sched, L.aux);
     return e;
 }

@@ -4,6 +4,25 @@
 
 namespace hb {
 
+// A launch with programmatic stream serialisation: the kernel may be scheduled
+// while the previous one of the stream drains; it starts with pdl_enter().
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, int block, int smem, cudaStream_t s,
+                              Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 struct ForceArgs {
     const void *pred;      // predicted slots, AoSoA32 (FP64 or mixed layout)
     int nchunk;            // number of 32-slot j chunks (padded slots / 32)
@@ -12,6 +31,7 @@ struct ForceArgs {
     double *force;         // [nact][F]
     double *partial;       // [S][gridDim.x*TI][F]  (only when S > 1)
     unsigned *counter;     // [gridDim.x], zero between launches
+    int deferred;          // the slices' partials are added by launch_reduce
     int *err;              // mapped host flag
     unsigned spin;         // poll limit of the waits for incoming tiles
                            // (kSpinLimit; lowered only by hb_set_wait_limit)
@@ -21,6 +41,11 @@ struct ForceArgs {
     double tsys;
     int nbody;
 };
+
+// Adds the S slice partials ([S][stride] doubles) of the first v values into
+// force, in a fixed order (hb_predict_pot.cu).  Chained to the force launch.
+cudaError_t launch_reduce(const double *partial, size_t stride, int S, int v, double *force,
+                          cudaStream_t s);
 
 // One compiled launch shape of the force kernel.
 struct ForceVariant {

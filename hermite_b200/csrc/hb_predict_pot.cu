@@ -22,6 +22,7 @@ predict_kernel(const double *__restrict__ jp, int n, int npad, double tsys,
     constexpr int R = Rec<ORDER>::words;
     __shared__ __align__(128) double rec[kPredThreads * R];
     __shared__ __align__(8) uint64_t bar;
+    pdl_enter();
     const int tid = threadIdx.x;
     const int base = blockIdx.x * kPredThreads;
     const int cnt = min(kPredThreads, n - base);
@@ -111,6 +112,51 @@ cudaError_t launch_predict(int order, bool mixed, const double *jp, int n, int n
     case 18: return launch_predict_t<9, false>(jp, n, npad, tsys, pred, err, s);
     }
     return cudaErrorInvalidValue;
+}
+
+// ---------------------------------------------------------------------------
+// Sum of the j-slices' partial forces (replaces reduce_kernel,
+// SRC/hermite4-titan.cu:303-327 and its 6th/8th-order counterparts).
+// A block takes 32 consecutive values and G groups of a warp each: group g adds slices
+// g, g + G, ... in 8 interleaved sums (8 loads in flight), combined pairwise;
+// the groups' sums are added in group order.
+template <int G>
+__global__ void __launch_bounds__(G * 32)
+reduce_kernel(const double *__restrict__ partial, size_t stride, int S, int v,
+              double *__restrict__ force)
+{
+    pdl_enter();
+    __shared__ double red[G][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int e = blockIdx.x * 32 + lane;
+    double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (e < v) {
+        const double *p = partial + e;
+        int s = g;
+        for (; s + 7 * G < S; s += 8 * G)
+#pragma unroll
+            for (int u = 0; u < 8; ++u) acc[u] += __ldcg(p + (size_t)(s + u * G) * stride);
+#pragma unroll
+        for (int u = 0; u < 7; ++u)
+            if (s + u * G < S) acc[u] += __ldcg(p + (size_t)(s + u * G) * stride);
+    }
+    red[g][lane] = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+    __syncthreads();
+    if (g == 0 && e < v) {
+        double sum = red[0][lane];
+#pragma unroll
+        for (int k = 1; k < G; ++k) sum += red[k][lane];
+        force[e] = sum;
+    }
+}
+
+cudaError_t launch_reduce(const double *partial, size_t stride, int S, int v, double *force,
+                          cudaStream_t s)
+{
+    const dim3 grid((v + 31) / 32);
+    if (S <= 16) return launch_pdl(reduce_kernel<2>, grid, 64, 0, s, partial, stride, S, v, force);
+    if (S <= 64) return launch_pdl(reduce_kernel<8>, grid, 256, 0, s, partial, stride, S, v, force);
+    return launch_pdl(reduce_kernel<32>, grid, 1024, 0, s, partial, stride, S, v, force);
 }
 
 // ---------------------------------------------------------------------------
