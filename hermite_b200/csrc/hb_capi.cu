@@ -666,9 +666,10 @@ int hb_potential(hb_ctx *ctx, double eps2, double *pot_out)
     if (!(eps2 >= 0.0)) return fail(ctx, HB_ERR_INVALID, "eps2 must be >= 0");
     int s = do_upload(ctx);
     if (s != HB_OK) return s;
-    HB_CK(launch_potential(ctx->order, ctx->d_jp, ctx->nbody, ctx->npad, eps2, ctx->d_posm,
-                           ctx->d_pot, ctx->d_err, ctx->stream));
-    ctx->launches += 2;
+    int launches = 0;
+    HB_CK(launch_potential(ctx->order, ctx->d_jp, ctx->nbody, ctx->npad, eps2, ctx->d_posm, ctx->d_pot,
+                           ctx->d_partial, ctx->partial_cap, ctx->nsm, ctx->d_err, ctx->stream, &launches));
+    ctx->launches += launches;
     HB_CK(cudaMemcpyAsync(ctx->h_pot, ctx->d_pot, sizeof(double) * ctx->nbody,
                           cudaMemcpyDeviceToHost, ctx->stream));
     s = sync_stream(ctx);
@@ -1176,11 +1177,12 @@ int hb_energy(hb_ctx *ctx, double eps2, double *kinetic, double *potential)
     int s = integrator_alloc(ctx);
     if (s == HB_OK) s = do_upload(ctx);
     if (s != HB_OK) return s;
-    HB_CK(launch_potential(ctx->order, ctx->d_jp, ctx->nbody, ctx->npad, eps2, ctx->d_posm,
-                           ctx->d_pot, ctx->d_err, ctx->stream));
+    int launches = 0;
+    HB_CK(launch_potential(ctx->order, ctx->d_jp, ctx->nbody, ctx->npad, eps2, ctx->d_posm, ctx->d_pot,
+                           ctx->d_partial, ctx->partial_cap, ctx->nsm, ctx->d_err, ctx->stream, &launches));
     HB_CK(integrator_energy(ctx->order, ctx->d_jp, ctx->d_pot, ctx->nbody, ctx->d_epart,
                             ctx->d_eout, ctx->stream));
-    ctx->launches += 4;
+    ctx->launches += launches + 2;
     s = sync_stream(ctx);
     if (s != HB_OK) return s;
     *kinetic = ctx->h_eout[0];

@@ -175,8 +175,10 @@ cudaError_t launch_force_lanes(int order, const ForceArgs &a, int nsm, cudaStrea
 
 cudaError_t launch_predict(int order, bool mixed, const double *jp, int n, int npad,
                            double tsys, void *pred, int *err, cudaStream_t s);
+// Potential of n slots; partial: scratch of cap doubles; *launches is advanced.
 cudaError_t launch_potential(int order, const double *jp, int n, int npad, double eps2,
-                             double *posm, double *pot, int *err, cudaStream_t s);
+                             double *posm, double *pot, double *partial, size_t cap, int nsm,
+                             int *err, cudaStream_t s, int *launches);
 cudaError_t run_fma_peak(int mode, int nsm, double *gflops);
 
 }  // namespace hb

@@ -1,4 +1,5 @@
 // hb_predict_pot.cu -- predictor, potential and the FMA-peak probe.
+#include <algorithm>
 #include <type_traits>
 #include "hb_internal.h"
 #include "hb_math.cuh"
@@ -175,6 +176,7 @@ template <int ORDER>
 __global__ void pack_posm_kernel(const double *__restrict__ jp, int n, int npad,
                                  double *__restrict__ posm)
 {
+    pdl_enter();
     constexpr int R = Rec<ORDER>::words, NC = posm_comps<ORDER>();
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= npad) return;
@@ -195,11 +197,14 @@ __global__ void pack_posm_kernel(const double *__restrict__ jp, int n, int npad,
 constexpr int kPotThreads = 128;
 constexpr int kPotTileChunks = 8;
 
+// j-slice blockIdx.y of gridDim.y writes its sums to row blockIdx.y of pot (row
+// stride `stride`).
 template <int NC>
 __global__ void __launch_bounds__(kPotThreads)
 potential_kernel(const double *__restrict__ posm, int nchunk, int n, double eps2,
-                 double *__restrict__ pot, int *err)
+                 double *__restrict__ pot, size_t stride, int *err)
 {
+    pdl_enter();
     constexpr int kPosmChunkBytes = NC * 32 * 8;
     constexpr int TB = kPotTileChunks * kPosmChunkBytes;
     __shared__ __align__(128) unsigned char ring[2 * TB];
@@ -214,7 +219,9 @@ potential_kernel(const double *__restrict__ posm, int nchunk, int n, double eps2
         yli = ci[160];
         zli = ci[192];
     }
-    const int ntile = (nchunk + kPotTileChunks - 1) / kPotTileChunks;
+    const int c0 = (int)((long long)blockIdx.y * nchunk / gridDim.y);
+    const int c1 = (int)((long long)(blockIdx.y + 1) * nchunk / gridDim.y);
+    const int ntile = (c1 - c0 + kPotTileChunks - 1) / kPotTileChunks;
 
     if (tid == 0) {
         mbar_init(&bar[0], 1);
@@ -223,11 +230,12 @@ potential_kernel(const double *__restrict__ posm, int nchunk, int n, double eps2
     }
     __syncthreads();
     auto issue = [&](int t) {
-        const int cnt = min(kPotTileChunks, nchunk - t * kPotTileChunks);
+        const int cnt = min(kPotTileChunks, c1 - c0 - t * kPotTileChunks);
         const uint32_t bytes = (uint32_t)(cnt * kPosmChunkBytes);
         mbar_arrive_expect_tx(&bar[t & 1], bytes);
         bulk_load(ring + (t & 1) * TB,
-                  reinterpret_cast<const unsigned char *>(posm) + (size_t)t * TB, bytes, &bar[t & 1]);
+                  reinterpret_cast<const unsigned char *>(posm) + (size_t)c0 * kPosmChunkBytes + (size_t)t * TB,
+                  bytes, &bar[t & 1]);
     };
     if (tid == 0) {
         issue(0);
@@ -244,11 +252,11 @@ potential_kernel(const double *__restrict__ posm, int nchunk, int n, double eps2
             }
             return;
         }
-        const int cnt = min(kPotTileChunks, nchunk - t * kPotTileChunks);
+        const int cnt = min(kPotTileChunks, c1 - c0 - t * kPotTileChunks);
         const double *tile = reinterpret_cast<const double *>(ring + (t & 1) * TB);
         for (int q = 0; q < cnt; ++q) {
             const double *cp = tile + q * NC * 32;
-            const int jbase = (t * kPotTileChunks + q) * 32;
+            const int jbase = (c0 + t * kPotTileChunks + q) * 32;
             double part = 0.0;
 #pragma unroll 8
             for (int jl = 0; jl < 32; ++jl) {
@@ -259,19 +267,240 @@ potential_kernel(const double *__restrict__ posm, int nchunk, int n, double eps2
                     dz = dz + (cp[192 + jl] - zli);
                 }
                 const double r2 = fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2)));
-                const double mj = (jbase + jl == i) ? 0.0 : cp[96 + jl];
-                part = fma(-mj, rsqrt_fp64(r2), part);
+                const double ri = (jbase + jl == i) ? 0.0 : rsqrt_fp64(r2);
+                part = fma(-cp[96 + jl], ri, part);
             }
             total += part;
         }
         __syncthreads();
         if (tid == 0 && t + 2 < ntile) issue(t + 2);
     }
-    if (i < n) pot[i] = total;
+    if (i < n) pot[blockIdx.y * stride + i] = total;
 }
 
+// Each pair once: a pair's rsqrt serves both particles (13 FP64 instructions
+// for two interactions instead of 24).
+//
+// Groups of 1024 slots (8 warps x 4 chunks of i-particles, one per lane and
+// chunk) meet every later chunk: lane l of a warp takes j = l + s of the chunk
+// in step s, the chunk's states and its running sums moving one lane per step
+// by shuffles (10 shuffles for 4 pairs, against 52 FP64 instructions).  So a
+// step adds to 4 i-sums and to one j-sum of every lane with no collisions, and
+// after 32 steps the j-sums are home.  The 8 warps' j-sums meet in shared
+// memory and go out once per (group, j).  The group's own chunks are summed
+// one-sided, as ordered pairs; the self pair is step 0 of a chunk with itself.
+//
+// A launch takes a band of groups, as many as `partial` has rows for, cut into
+// slices of `lc` chunks; pot_band_kernel then adds rows and slices to the
+// potentials in a fixed order, so results are deterministic.
+//
+// N = 100003: 5.27 ms (11.0 ms with ordered pairs and no slices), 65 % of the
+// FP64 pipe's rate on the 13 instructions per pair; 8 i-chunks a warp, 2 of
+// 16 warps, three CTAs per SM and other unrollings measured 0-10 % slower.
+constexpr int kSymWarps = 8, kSymI = 4, kSymTile = 16;
+constexpr int kSymChunks = kSymWarps * kSymI, kSymSlots = kSymChunks * 32;
+
+struct PotBand {
+    const double *posm;
+    double *rows, *cols;   // j-sums [group][npad]; i-sums [group][smax][kSymSlots]
+    int g0, ng, smax, lc, nchunk;
+    double eps2;
+    int *err;
+};
+
+__host__ __device__ __forceinline__ int pot_slices(int nchunk, int g, int lc)
+{
+    return (nchunk - g * kSymChunks + lc - 1) / lc;
+}
+
+template <bool DIAG>
+__device__ __forceinline__ void pot_chunk(const double *cp, int lane, const double (&xi)[kSymI][3],
+                                          const double (&mi)[kSymI], const bool (&own)[kSymI],
+                                          double eps2, double (&total)[kSymI], double &fj)
+{
+    double x = cp[lane], y = cp[32 + lane], z = cp[64 + lane], m = cp[96 + lane];
+    double part[kSymI];
+#pragma unroll
+    for (int k = 0; k < kSymI; ++k) part[k] = 0.0;
+    fj = 0.0;
+    const int next = (lane + 1) & 31;
+#pragma unroll 4
+    for (int s = 0; s < 32; ++s) {
+#pragma unroll
+        for (int k = 0; k < kSymI; ++k) {
+            const double dx = x - xi[k][0], dy = y - xi[k][1], dz = z - xi[k][2];
+            double ri = rsqrt_fp64(fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))));
+            if (DIAG && s == 0 && own[k]) ri = 0.0;
+            part[k] = fma(-m, ri, part[k]);
+            if (!DIAG) fj = fma(-mi[k], ri, fj);
+        }
+        x = __shfl_sync(0xffffffffu, x, next);
+        y = __shfl_sync(0xffffffffu, y, next);
+        z = __shfl_sync(0xffffffffu, z, next);
+        m = __shfl_sync(0xffffffffu, m, next);
+        if (!DIAG) fj = __shfl_sync(0xffffffffu, fj, next);
+    }
+#pragma unroll
+    for (int k = 0; k < kSymI; ++k) total[k] += part[k];
+}
+
+__global__ void __launch_bounds__(kSymWarps * 32, 2)
+potential_sym_kernel(const PotBand a)
+{
+    pdl_enter();
+    constexpr int CB = 4 * 32 * 8, TB = kSymTile * CB, T = kSymWarps * 32;
+    extern __shared__ __align__(128) unsigned char smem[];
+    double *accj = reinterpret_cast<double *>(smem + 2 * TB);      // [warp][tile chunk][32]
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + 2 * TB + kSymWarps * kSymTile * 32 * 8);
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    int g = a.g0, s = blockIdx.x;
+    while (s >= pot_slices(a.nchunk, g, a.lc)) s -= pot_slices(a.nchunk, g++, a.lc);
+    const int own0 = g * kSymChunks, own1 = min(own0 + kSymChunks, a.nchunk);
+    const int c0 = own0 + s * a.lc, c1 = min(c0 + a.lc, a.nchunk);
+
+    double xi[kSymI][3], mi[kSymI], total[kSymI];
+#pragma unroll
+    for (int k = 0; k < kSymI; ++k) {
+        const int ci = own0 + w * kSymI + k;
+        const double *p = a.posm + (size_t)min(ci, a.nchunk - 1) * 4 * 32 + lane;
+        for (int d = 0; d < 3; ++d) xi[k][d] = p[d * 32];
+        mi[k] = ci < a.nchunk ? p[96] : 0.0;       // past the last chunk: adds nothing
+        total[k] = 0.0;
+    }
+    if (tid == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    const int ntile = (c1 - c0 + kSymTile - 1) / kSymTile;
+    auto issue = [&](int t) {
+        const uint32_t bytes = (uint32_t)(min(kSymTile, c1 - c0 - t * kSymTile) * CB);
+        mbar_arrive_expect_tx(&bar[t & 1], bytes);
+        bulk_load(smem + (t & 1) * TB, a.posm + (size_t)(c0 + t * kSymTile) * 4 * 32, bytes, &bar[t & 1]);
+    };
+    if (tid == 0) {
+        issue(0);
+        if (ntile > 1) issue(1);
+    }
+    for (int t = 0; t < ntile; ++t) {
+        const bool got = mbar_wait_bounded(&bar[t & 1], (uint32_t)((t >> 1) & 1));
+        if (!__syncthreads_and(got)) {
+            if (tid == 0) {
+                raise_error(a.err, kErrWaitTimeout);
+                for (int u = t; u < ntile && u < t + 2; ++u)
+                    mbar_wait_bounded(&bar[u & 1], (uint32_t)((u >> 1) & 1));
+            }
+            return;
+        }
+        // lc and the groups are whole tiles: a tile is in the group or past it
+        const int ct = c0 + t * kSymTile, cnt = min(kSymTile, c1 - ct);
+        const double *tile = reinterpret_cast<const double *>(smem + (t & 1) * TB);
+        const bool diag = ct < own1;
+        for (int q = 0; q < cnt; ++q) {
+            double fj;
+            bool own[kSymI];
+            if (diag) {
+#pragma unroll
+                for (int k = 0; k < kSymI; ++k) own[k] = ct + q == own0 + w * kSymI + k;
+                pot_chunk<true>(tile + q * 4 * 32, lane, xi, mi, own, a.eps2, total, fj);
+            } else {
+                pot_chunk<false>(tile + q * 4 * 32, lane, xi, mi, own, a.eps2, total, fj);
+                accj[(w * kSymTile + q) * 32 + lane] = fj;
+            }
+        }
+        __syncthreads();
+        if (tid == 0 && t + 2 < ntile) issue(t + 2);
+        if (!diag) {
+            double *row = a.rows + (size_t)(g - a.g0) * a.nchunk * 32 + (size_t)ct * 32;
+            for (int e = tid; e < cnt * 32; e += T) {
+                double v = accj[e];
+#pragma unroll
+                for (int ww = 1; ww < kSymWarps; ++ww) v += accj[ww * kSymTile * 32 + e];
+                row[e] = v;
+            }
+            __syncthreads();
+        }
+    }
+    double *col = a.cols + ((size_t)(g - a.g0) * a.smax + s) * kSymSlots;
+#pragma unroll
+    for (int k = 0; k < kSymI; ++k) col[(w * kSymI + k) * 32 + lane] = total[k];
+}
+
+// Adds a band's sums to the potentials of the slots from its first group on.
+__global__ void __launch_bounds__(256)
+pot_band_kernel(const PotBand a, int n, double *__restrict__ pot)
+{
+    pdl_enter();
+    const int j = a.g0 * kSymSlots + blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n) return;
+    const int gj = j / kSymSlots, before = min(gj - a.g0, a.ng);   // groups below j's own
+    double acc[8] = {a.g0 > 0 ? pot[j] : 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    auto add = [&](const double *p, size_t stride, int cnt) {
+        int k = 0;
+        for (; k + 8 <= cnt; k += 8)
+#pragma unroll
+            for (int u = 0; u < 8; ++u) acc[u] += __ldcg(p + (size_t)(k + u) * stride);
+#pragma unroll
+        for (int u = 0; u < 7; ++u)
+            if (k + u < cnt) acc[u] += __ldcg(p + (size_t)(k + u) * stride);
+    };
+    add(a.rows + j, (size_t)a.nchunk * 32, before);
+    if (gj - a.g0 < a.ng)
+        add(a.cols + (size_t)(gj - a.g0) * a.smax * kSymSlots + j % kSymSlots, kSymSlots,
+            pot_slices(a.nchunk, gj, a.lc));
+    pot[j] = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+}
+
+// Each-pair-once potential in bands; *launches counts them.  Returns
+// cudaErrorInvalidValue when `cap` doubles hold no band of one group.
+static cudaError_t launch_potential_sym(int n, int npad, double eps2, const double *posm, double *pot,
+                                        double *partial, size_t cap, int nsm, int *err,
+                                        cudaStream_t s, int *launches)
+{
+    constexpr int smem = 2 * kSymTile * 4 * 32 * 8 + kSymWarps * kSymTile * 32 * 8 + 16;
+    cudaError_t e = cudaFuncSetAttribute(potential_sym_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    PotBand a{};
+    a.posm = posm;
+    a.nchunk = npad / 32;
+    a.eps2 = eps2;
+    a.err = err;
+    const int groups = (a.nchunk + kSymChunks - 1) / kSymChunks;
+    for (int g0 = 0; g0 < groups; g0 += a.ng) {
+        // about 8 waves of two CTAs per SM: a CTA's chunks, in whole tiles
+        const long long wide = std::min((long long)groups - g0, (long long)(cap / npad));
+        const long long units = std::max(1LL, wide) * (a.nchunk - (long long)g0 * kSymChunks);
+        const long long lc = units / (16LL * nsm);
+        a.g0 = g0;
+        a.lc = (int)std::max(1LL, (lc + kSymTile - 1) / kSymTile) * kSymTile;
+        a.smax = pot_slices(a.nchunk, g0, a.lc);
+        const long long per = (long long)npad + (long long)a.smax * kSymSlots;
+        a.ng = (int)std::min((long long)(groups - g0), (long long)cap / per);
+        if (a.ng < 1) return cudaErrorInvalidValue;
+        a.rows = partial;
+        a.cols = partial + (size_t)a.ng * npad;
+        int ctas = 0;
+        for (int g = g0; g < g0 + a.ng; ++g) ctas += pot_slices(a.nchunk, g, a.lc);
+        e = launch_pdl(potential_sym_kernel, dim3(ctas), kSymWarps * 32, smem, s, a);
+        if (e == cudaSuccess)
+            e = launch_pdl(pot_band_kernel, dim3((n - g0 * kSymSlots + 255) / 256), 256, 0, s, a, n, pot);
+        if (e != cudaSuccess) return e;
+        *launches += 2;
+    }
+    return cudaSuccess;
+}
+
+// From this many slots on the pairs are taken once: 16384: 191 against 283 us
+// with ordered pairs, 100003: 5.27 against 8.90 ms, 262144: 34.3 against 60.8;
+// 12000: 189 against 171 us, too few groups to fill the GPU evenly.
+// Double-double positions keep the ordered pairs.
+constexpr int kPotSymMin = 14336;
+
 cudaError_t launch_potential(int order, const double *jp, int n, int npad, double eps2,
-                             double *posm, double *pot, int *err, cudaStream_t s)
+                             double *posm, double *pot, double *partial, size_t cap, int nsm,
+                             int *err, cudaStream_t s, int *launches)
 {
     const int g = npad / 128;
     switch (order) {
@@ -283,11 +512,26 @@ cudaError_t launch_potential(int order, const double *jp, int n, int npad, doubl
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
+    ++*launches;
+    if (order != 9 && n >= kPotSymMin && (size_t)npad * 2 <= cap)
+        return launch_potential_sym(n, npad, eps2, posm, pot, partial, cap, nsm, err, s, launches);
+    // j-slices of at least one tile, about 4 waves of 12 CTAs per SM
+    const int nchunk = npad / 32, gx = npad / kPotThreads;
+    int S = std::max(1, std::min(nchunk / kPotTileChunks, 48 * nsm / gx));
+    S = (int)std::min<size_t>(S, cap / npad);
+    S = std::max(S, 1);
+    double *out = S > 1 ? partial : pot;
     if (order == 9)
-        potential_kernel<7><<<npad / kPotThreads, kPotThreads, 0, s>>>(posm, npad / 32, n, eps2, pot, err);
+        e = launch_pdl(potential_kernel<7>, dim3(gx, S), kPotThreads, 0, s, (const double *)posm, nchunk, n,
+                       eps2, out, (size_t)npad, err);
     else
-        potential_kernel<4><<<npad / kPotThreads, kPotThreads, 0, s>>>(posm, npad / 32, n, eps2, pot, err);
-    return cudaGetLastError();
+        e = launch_pdl(potential_kernel<4>, dim3(gx, S), kPotThreads, 0, s, (const double *)posm, nchunk, n,
+                       eps2, out, (size_t)npad, err);
+    if (e != cudaSuccess) return e;
+    ++*launches;
+    if (S == 1) return cudaSuccess;
+    ++*launches;
+    return launch_reduce(partial, (size_t)npad, S, n, pot, s);
 }
 
 // ---------------------------------------------------------------------------
