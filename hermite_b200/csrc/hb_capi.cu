@@ -308,11 +308,11 @@ int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
         a.eps2 = eps2;
         a.force = force_out_dev;
         a.partial = ctx->d_partial;
-        a.counter = ctx->d_counter;
         a.err = ctx->d_err;
         a.spin = ctx->wait_limit;
-        HB_CK(launch_force_lanes(ctx->order, a, ctx->nsm, ctx->stream));
-        ctx->launches++;
+        int launches = 0;
+        HB_CK(launch_force_lanes(ctx->order, a, ctx->nsm, ctx->stream, &launches));
+        ctx->launches += launches;
         return HB_OK;
     }
     const bool automatic = ctx->variant_override < 0 && ctx->jsplit_override == 0;

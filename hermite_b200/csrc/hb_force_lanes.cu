@@ -13,9 +13,15 @@
 // sums meet in a fixed xor-shuffle tree.  The warps of a CTA take the chunks
 // of its j-slice in turn; each warp brings its chunks' raw records into shared
 // memory by bulk copies, two in flight (every wait bounded), and predicts them
-// there (one lane per slot), so a launch reads every j record once.  The CTAs of the grid are j-slices; the last one to finish
-// adds the slices' partials, spread over its threads.  Every sum has a fixed
+// there (one lane per slot), so a launch reads every j record once.  The CTAs of
+// the grid are j-slices, added by a chained reduce launch.  Every sum has a fixed
 // association for a given (nact, N), so results are deterministic.
+//
+// Measured at 6th order, N = 262144, back to back: nact = 1 / 4 / 16 take 11.1 /
+// 14.5 / 25.5 us.  With the slices added by the last CTA (up to 37 rounds of
+// loads in turn) and records read word by word (4-way bank conflicts) they
+// took 14.5 / 18.5 / 37.6.  8th order, N = 2^20, nact = 1: 37.9 us, of which the
+// records take 33.8 at the measured HBM copy rate.
 //
 // The same job as the reference's force_kernel with its j-blocks
 // (SRC/hermite4-titan.cu:189-238, SRC/hermite6-titan.cu:245-299,
@@ -35,7 +41,7 @@ constexpr int kLanesStages = 2;     // raw chunks in flight per warp
 // Dynamic shared memory of one CTA: per warp, kLanesStages raw chunks (32
 // records each, AoS, filled by bulk copies) and one predicted chunk; then
 // the warps' mbarriers.  After the j loop the front of it holds the warps'
-// group sums and then the cross-slice group sums.
+// group sums.
 template <int ORDER>
 struct LanesSmem {
     static constexpr int raw = 32 * Rec<ORDER>::bytes;        // 3584 / 5120 / 6656
@@ -45,8 +51,58 @@ struct LanesSmem {
     static constexpr int bytes = bar_off + kLanesWarps * kLanesStages * 8;
     static_assert(raw % 16 == 0 && pred % 16 == 0, "bulk copies need 16-byte offsets");
     static_assert(bar_off >= kLanesWarps * kLanesMaxAct * Frc<ORDER>::words * 8, "reduction space");
-    static_assert(bar_off >= 2 * kLanesWarps * 32 * 8, "slice sums");
 };
+
+// A lane's raw record from a chunk in shared memory, 16 bytes a load (records
+// are 14, 20 or 26 words).  20-word records lie 160 bytes apart, so lanes l and
+// l + 4 of a quarter warp meet in the same banks: lanes 4..7 take every two
+// loads in the other order.  Loading word by word cost 160 shared-memory cycles a
+// 6th-order chunk; this costs 40.
+template <int ORDER>
+__device__ __forceinline__ void load_record(const double *raw, int lane, double *r)
+{
+    constexpr int R = Rec<ORDER>::words;
+    static_assert(R % 2 == 0, "16-byte records");
+    const double2 *p = reinterpret_cast<const double2 *>(raw + lane * R);
+    if constexpr (R % 4 == 0) {
+        const int swap = (lane >> 2) & 1;
+#pragma unroll
+        for (int k = 0; k < R / 2; k += 2) {
+            const double2 a = p[k + swap], b = p[k + 1 - swap];
+            r[2 * k] = swap ? b.x : a.x;
+            r[2 * k + 1] = swap ? b.y : a.y;
+            r[2 * k + 2] = swap ? a.x : b.x;
+            r[2 * k + 3] = swap ? a.y : b.y;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < R / 2; ++k) {
+            const double2 a = p[k];
+            r[2 * k] = a.x;
+            r[2 * k + 1] = a.y;
+        }
+    }
+}
+
+template <int ORDER>
+__device__ __forceinline__ void predict_lane(const double *raw, int chunk, int nbody, double tsys,
+                                             Body64 &b)
+{
+    const int lane = threadIdx.x & 31, slot = chunk * 32 + lane;
+    if (slot < nbody) {
+        double r[Rec<ORDER>::words];
+        load_record<ORDER>(raw, lane, r);
+        predict_slot<ORDER>(r, tsys, b.x, b.v, b.a, b.jk);
+        b.m = r[3];
+    } else {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            b.x[k] = pad_position(slot, k);
+            b.v[k] = b.a[k] = b.jk[k] = 0.0;
+        }
+        b.m = 0.0;
+    }
+}
 
 // Predicts the 32 slots of chunk `chunk` (one per lane) from their raw
 // records in shared memory into the predicted FP64 chunk layout at dst.  Out
@@ -56,28 +112,21 @@ template <int ORDER>
 __device__ __noinline__ void predict_raw_chunk(const double *raw, int chunk, int nbody,
                                                double tsys, double *dst)
 {
-    constexpr int R = Rec<ORDER>::words;
-    const int lane = threadIdx.x & 31, slot = chunk * 32 + lane;
-    double x[3], v[3], ac[3] = {0.0, 0.0, 0.0}, jk[3] = {0.0, 0.0, 0.0}, m;
-    if (slot < nbody) {
-        const double *r = raw + lane * R;
-        predict_slot<ORDER>(r, tsys, x, v, ac, jk);
-        m = r[3];
-    } else {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) { x[k] = pad_position(slot, k); v[k] = 0.0; }
-        m = 0.0;
-    }
+    const int lane = threadIdx.x & 31;
+    Body64 b;
+    predict_lane<ORDER>(raw, chunk, nbody, tsys, b);
     double *c = dst + lane;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        c[(P64_X + k) * 32] = x[k];
-        c[(P64_V + k) * 32] = v[k];
-        if constexpr (ORDER >= 6) c[(P64_A + k) * 32] = ac[k];
-        if constexpr (ORDER >= 8) c[(P64_J + k) * 32] = jk[k];
+        c[(P64_X + k) * 32] = b.x[k];
+        c[(P64_V + k) * 32] = b.v[k];
+        if constexpr (ORDER >= 6) c[(P64_A + k) * 32] = b.a[k];
+        if constexpr (ORDER >= 8) c[(P64_J + k) * 32] = b.jk[k];
     }
-    c[P64_M * 32] = m;
+    c[P64_M * 32] = b.m;
 }
+
+__device__ __forceinline__ double from_lane0(double v) { return __shfl_sync(0xffffffffu, v, 0); }
 
 template <int ORDER, int LOG2G>
 __global__ void __launch_bounds__(kLanesWarps * 32)
@@ -86,8 +135,8 @@ force_lanes_kernel(ForceArgs a)
     using L = LanesSmem<ORDER>;
     constexpr int G = 1 << LOG2G, STG = kLanesStages;
     constexpr int F = Frc<ORDER>::words, R = Rec<ORDER>::words;
+    pdl_enter();
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ unsigned s_last;
     __shared__ int s_fail;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int p = lane >> LOG2G, g = lane & (G - 1);
@@ -127,6 +176,27 @@ force_lanes_kernel(ForceArgs a)
         const int st = q % STG;
         const bool got = mbar_wait_bounded(&bar[st], (uint32_t)((q / STG) & 1), a.spin);
         if (!__all_sync(0xffffffffu, got)) { failed_at = q; break; }
+        if constexpr (LOG2G == 5) {
+            // one i-particle: every lane keeps the j it predicts in registers;
+            // this one copy of the code serves i (chunk 0, lane 0) and j
+            Body64 J;
+            predict_lane<ORDER>(reinterpret_cast<const double *>(wraw + st * L::raw), chunk_of(q),
+                                a.nbody, a.tsys, J);
+            __syncwarp();                // the raw stage is read: refill it
+            if (lane == 0 && q + STG < nload) issue(q + STG);
+            if (q == 0) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    I.x[k] = from_lane0(J.x[k]);
+                    I.v[k] = from_lane0(J.v[k]);
+                    if constexpr (ORDER >= 6) I.a[k] = from_lane0(J.a[k]);
+                    if constexpr (ORDER >= 8) I.jk[k] = from_lane0(J.jk[k]);
+                }
+            } else {
+                interact64<ORDER>(I, J, a.eps2, f);
+            }
+            continue;
+        }
         predict_raw_chunk<ORDER>(reinterpret_cast<const double *>(wraw + st * L::raw), chunk_of(q),
                                  a.nbody, a.tsys, my);
         __syncwarp();                    // the raw stage is read: refill it
@@ -169,38 +239,6 @@ force_lanes_kernel(ForceArgs a)
         if (S == 1) a.force[e] = v;
         else a.partial[(size_t)sl * kLanesMaxAct * F + e] = v;
     }
-    if (S == 1) return;
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) s_last = atomicAdd(&a.counter[0], 1u) == (unsigned)(S - 1);
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    // the slices' sum, spread over the CTA: thread t = k*V + e adds slices
-    // k, k+K, ... of value e into 8 interleaved sums (8 loads in flight),
-    // combined pairwise; then each value's K group sums in group order
-    const int K = max(1, (int)blockDim.x / V);
-    double *grp = reinterpret_cast<double *>(smem);
-    for (int t = tid; t < K * V; t += blockDim.x) {
-        const int k = t / V, e = t - k * V;
-        double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        int s2 = k;
-        for (; s2 + 7 * K < S; s2 += 8 * K)
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                acc[u] += __ldcg(a.partial + (size_t)(s2 + u * K) * kLanesMaxAct * F + e);
-#pragma unroll
-        for (int u = 0; u < 7; ++u)
-            if (s2 + u * K < S) acc[u] += __ldcg(a.partial + (size_t)(s2 + u * K) * kLanesMaxAct * F + e);
-        grp[t] = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
-    }
-    __syncthreads();
-    for (int e = tid; e < V; e += blockDim.x) {
-        double v = grp[e];
-        for (int k = 1; k < K; ++k) v += grp[k * V + e];
-        a.force[e] = v;
-    }
-    if (tid == 0) a.counter[0] = 0u;
 }
 
 }  // namespace
@@ -251,7 +289,7 @@ cudaError_t lanes_setup(int oi, int *per_sm)
 
 }  // namespace
 
-cudaError_t launch_force_lanes(int order, const ForceArgs &a, int nsm, cudaStream_t s)
+cudaError_t launch_force_lanes(int order, const ForceArgs &a, int nsm, cudaStream_t s, int *launches)
 {
     static_assert(kLanesMaxAct <= 16, "one lane per i-particle is the tiled kernel's job");
     if (a.nact < 1 || a.nact > kLanesMaxAct || a.nchunk < 1) return cudaErrorInvalidValue;
@@ -263,8 +301,13 @@ cudaError_t launch_force_lanes(int order, const ForceArgs &a, int nsm, cudaStrea
     const int log2g = lanes_log2g(a.nact);                // P = 2^(5 - log2g) >= nact, G >= 2
     // j-slices of at least two chunks a warp, all CTAs resident at once
     const int S = std::max(1, std::min(std::min(2, per_sm) * nsm, a.nchunk / (2 * kLanesWarps)));
-    kLanesTable[oi][log2g - 1]<<<S, kLanesWarps * 32, kLanesBytes[oi], s>>>(a);
-    return cudaGetLastError();
+    const int F = 3 * (order / 2);
+    e = launch_pdl(kLanesTable[oi][log2g - 1], dim3(S), kLanesWarps * 32, kLanesBytes[oi], s, a);
+    if (e != cudaSuccess) return e;
+    ++*launches;
+    if (S == 1) return cudaSuccess;
+    ++*launches;
+    return launch_reduce(a.partial, (size_t)kLanesMaxAct * F, S, a.nact * F, a.force, s);
 }
 
 }  // namespace hb
