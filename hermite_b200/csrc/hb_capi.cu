@@ -38,8 +38,9 @@ namespace {
 constexpr int kMaxBody = 1 << 24;
 // hb_set_jp_records of at least this many bytes uploads at once, in chunks.
 constexpr size_t kEagerUploadBytes = (size_t)4 << 20, kUploadChunkBytes = (size_t)2 << 20;
-// HB_ENGINE_AUTO takes the team engine up to this many particles.
-constexpr int kTeamAutoMaxBody = 3072;
+// HB_ENGINE_AUTO takes the team engine up to this many particles (4th order, us
+// per block step, team against graph: N = 2048 9.7 / 11.9, 2500 11.7 / 12.3, 3000 17.7 / 13.8).
+constexpr int kTeamAutoMaxBody = 2560;
 
 int rec_words(int order) { return 8 + 3 * (order - 2); }
 int force_words(int order) { return 3 * (order / 2); }
@@ -79,7 +80,7 @@ struct hb_ctx {
     Sched *h_sched = nullptr;       // host copy of the scheduler (set-up only)
     Sched *d_sched = nullptr;       // device scheduler
     IntStatus *h_status = nullptr, *d_status = nullptr;   // mapped pinned
-    double *d_dt = nullptr;
+    double *d_dt = nullptr, *d_tn = nullptr;
     int *d_ilist = nullptr;
     double *d_epart = nullptr, *h_eout = nullptr, *d_eout = nullptr;
     cudaGraph_t int_graph = nullptr;
@@ -93,7 +94,7 @@ struct hb_ctx {
     int *d_team_next = nullptr;
     // persistent engine
     unsigned *d_gbar = nullptr;       // grid barrier words, zero between launches
-    IntegratorLaunch int_L{};         // the step's buffers and work-item target
+    IntegratorLaunch int_L{};         // the step's buffers
     int persist_grid = 0;             // resident CTAs of the persistent kernel
     int blocks_per_sm[2][kNumVariants] = {};
     bool smem_set[2][kNumVariants] = {};
@@ -440,6 +441,7 @@ int hb_destroy(hb_ctx *ctx)
     cudaFreeHost(ctx->h_status);
     cudaFreeHost(ctx->h_eout);
     cudaFree(ctx->d_dt);
+    cudaFree(ctx->d_tn);
     cudaFree(ctx->d_ilist);
     cudaFree(ctx->d_epart);
     cudaFree(ctx->d_team_sys);
@@ -762,7 +764,7 @@ int hb_force_variant_info(int order, int precision, int variant, int *threads, i
 
 // ---- device-resident integration -------------------------------------------
 namespace {
-constexpr int kStepsPerGraph = 32;
+constexpr int kStepsPerGraph = 32;      // even: the steps' two counters take turns
 constexpr int kEnergyParts = 256;
 
 int integrator_alloc(hb_ctx *ctx)
@@ -775,6 +777,7 @@ int integrator_alloc(hb_ctx *ctx)
               cudaHostAlloc((void **)&ctx->h_eout, 2 * sizeof(double), cudaHostAllocMapped) == cudaSuccess &&
               cudaHostGetDevicePointer((void **)&ctx->d_eout, ctx->h_eout, 0) == cudaSuccess &&
               cudaMalloc((void **)&ctx->d_dt, np * sizeof(double)) == cudaSuccess &&
+              cudaMalloc((void **)&ctx->d_tn, np * sizeof(double)) == cudaSuccess &&
               cudaMalloc((void **)&ctx->d_ilist, np * sizeof(int)) == cudaSuccess &&
               cudaMalloc((void **)&ctx->d_epart, 2 * kEnergyParts * sizeof(double)) == cudaSuccess &&
               cudaMalloc((void **)&ctx->d_aux, np * kAuxWords * sizeof(double)) == cudaSuccess &&
@@ -800,7 +803,6 @@ int setup_integrator(hb_ctx *ctx, double tsys, double eps2, double eta, double d
 {
     Sched &sc = *ctx->h_sched;
     std::memset(&sc, 0, sizeof(Sched));
-    sc.tnext_bits = 0x7ff0000000000000ull;
     sc.tsys = tsys;
     sc.tend = tsys;
     sc.eps2 = eps2;
@@ -818,37 +820,33 @@ int setup_integrator(hb_ctx *ctx, double tsys, double eps2, double eta, double d
     const TeamSys ts{0, ctx->nbody, 0, eps2};
     HB_CK(cudaMemcpy(ctx->d_team_sys, &ts, sizeof(TeamSys), cudaMemcpyHostToDevice));
 
-    IntegratorLaunch L;
+    IntegratorLaunch L{};
     L.jp = ctx->d_jp;
     L.dt = ctx->d_dt;
+    L.tn = ctx->d_tn;
     L.aux = ctx->d_aux;
+    L.pred = ctx->d_pred;
     L.ilist = ctx->d_ilist;
     L.sched = ctx->d_sched;
     L.force = ctx->d_force;
     L.partial = ctx->d_partial;
-    L.counter = ctx->d_counter;
     L.err = ctx->d_err;
     L.n = ctx->nbody;
     L.nchunk = ctx->npad / 32;
     L.nsm = ctx->nsm;
     L.partial_cap = ctx->partial_cap;
     L.mixed = ctx->precision == HB_MIXED;
-    int smem = 0, per_sm = 0, big_per_sm = 0;
-    HB_CK(integrator_kernel_setup(ctx->order, L.mixed, &smem, &per_sm, &big_per_sm));
-    L.smem_fp64 = L.smem_mixed = smem;
-    L.items_grid = ctx->nsm * std::max(1, per_sm);
-    L.big_grid = ctx->nsm * std::max(1, big_per_sm);
-    L.target_items = 2 * L.items_grid;
+    HB_CK(integrator_kernel_setup(ctx->order, L.mixed));
     ctx->int_L = L;
-    int psmem = 0, p_per_sm = 0;
-    HB_CK(persistent_setup(ctx->order, L.mixed, &psmem, &p_per_sm));
+    int p_per_sm = 0;
+    HB_CK(persistent_setup(ctx->order, L.mixed, &p_per_sm));
     ctx->persist_grid = ctx->nsm * p_per_sm;
 
     if (ctx->stream == nullptr) return fail(ctx, HB_ERR_STATE, "integrator needs a non-default stream");
     HB_CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t ce = cudaSuccess;
     for (int k = 0; k < kStepsPerGraph && ce == cudaSuccess; ++k)
-        ce = integrator_step_launch(ctx->order, L, ctx->stream);
+        ce = integrator_step_launch(ctx->order, L, k & 1, ctx->stream);
     cudaGraph_t graph = nullptr;
     const cudaError_t ee = cudaStreamEndCapture(ctx->stream, &graph);
     if (ce != cudaSuccess || ee != cudaSuccess) {
@@ -1138,6 +1136,9 @@ int hb_integrator_run(hb_ctx *ctx, double tend, long long max_block_steps)
     const int engine = resolve_engine(ctx, &cfg);
     if (engine < 0) return -engine;
     if (engine == HB_ENGINE_TEAM) return run_team(ctx, cfg, tend, max_block_steps);
+    ctx->pred_stale = true;          // the steps predict into the same array
+    HB_CK(integrator_start(ctx->order, ctx->int_L, ctx->stream));
+    ctx->launches += 2;
     if (engine == HB_ENGINE_PERSISTENT) return run_persistent(ctx, tend, max_block_steps);
     long long last_steps = st->block_steps;
     const long long first_steps = st->block_steps;
@@ -1146,7 +1147,7 @@ int hb_integrator_run(hb_ctx *ctx, double tend, long long max_block_steps)
             return fail(ctx, HB_ERR_STATE, "block-step limit %lld reached at t = %.17g",
                         max_block_steps, st->tsys);
         HB_CK(cudaGraphLaunch(ctx->int_exec, ctx->stream));
-        ctx->launches += 5LL * kStepsPerGraph;
+        ctx->launches += 3LL * kStepsPerGraph;
         s = sync_stream(ctx);
         if (s != HB_OK) return s;
         if (st->error)

@@ -45,6 +45,23 @@ __device__ __forceinline__ double norm2(V3 a)
     return __dadd_rn(__dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y)), __dmul_rn(a.z, a.z));
 }
 
+// calc_dtlim (SRC/nbodysystem.h:652-661): dtmax halved until tnext is a
+// multiple of it, at most 64 times.  For a power-of-two dtmax = 2^D this is
+// 2^(D-k) with k = clamp(D - e, 0, 64), e the exponent of the lowest set
+// bit of tnext (tnext = 0 is a multiple of everything): the same value the
+// reference's loop reaches, from the exponent and significand bits.
+__device__ __forceinline__ double calc_dtlim(double tnext, double dtmax)
+{
+    if (!(tnext > 0.0)) return dtmax;
+    const long long b = __double_as_longlong(tnext);
+    const int ex = (int)((b >> 52) & 0x7ff);
+    const long long sig = (b & 0xfffffffffffffll) | (ex ? (1ll << 52) : 0ll);
+    const int e = (ex ? ex : 1) - 1075 + (__ffsll(sig) - 1);
+    const int D = (int)((__double_as_longlong(dtmax) >> 52) & 0x7ff) - 1023;
+    const int k = max(0, min(64, D - e));
+    return __longlong_as_double(__double_as_longlong(dtmax) - ((long long)k << 52));
+}
+
 // Particle state in a j-particle record r (pos mass vel tlast acc jrk [snp
 // crk] [d4a d5a] [posL]); f = the new force (acc jrk [snp] [crk]).  ORDER 9
 // is the 8th-order corrector with double-double positions

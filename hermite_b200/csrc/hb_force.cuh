@@ -53,6 +53,39 @@ struct ForceShape {
     static_assert(!FUSED || TI <= TCH * 32, "fused: the i-tile must fit one raw stage");
 };
 
+// Writes one predicted state into its column of an AoSoA32 chunk (FP64 or
+// hi/lo mixed); col: the chunk's address plus the lane.
+template <int ORDER, bool MIXED>
+__device__ __forceinline__ void put_predicted(void *col, const double (&x)[3], const double (&v)[3],
+                                              const double (&a)[3], const double (&jk)[3],
+                                              const double (&xl)[3], double m)
+{
+    if constexpr (MIXED) {
+        float *c = static_cast<float *>(col);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float hi = __double2float_rn(x[k]);
+            c[(PMX_XH + k) * 32] = hi;
+            c[(PMX_XL + k) * 32] = __double2float_rn(x[k] - (double)hi);
+            c[(PMX_V + k) * 32] = __double2float_rn(v[k]);
+            if constexpr (ORDER >= 6) c[(PMX_A + k) * 32] = __double2float_rn(a[k]);
+            if constexpr (ORDER == 8) c[(PMX_J + k) * 32] = __double2float_rn(jk[k]);
+        }
+        c[PMX_M * 32] = __double2float_rn(m);
+    } else {
+        double *c = static_cast<double *>(col);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            c[(P64_X + k) * 32] = x[k];
+            c[(P64_V + k) * 32] = v[k];
+            if constexpr (ORDER >= 6) c[(P64_A + k) * 32] = a[k];
+            if constexpr (ORDER >= 8) c[(P64_J + k) * 32] = jk[k];
+            if constexpr (ORDER == 9) c[(P64_XL + k) * 32] = xl[k];
+        }
+        c[P64_M * 32] = m;
+    }
+}
+
 // Predicts nslot consecutive records (raw, AoS) to tsys into the predicted
 // AoSoA32 layout at `out` (FP64 or hi/lo mixed), slots >= n as padding.
 // One out-of-line copy serves both the i- and the j-particles of the fused
@@ -74,33 +107,8 @@ __device__ __noinline__ void predict_tile(const double *raw, int nslot, int slot
             for (int k = 0; k < 3; ++k) { x[k] = pad_position(slot, k); v[k] = 0.0; }
             m = 0.0;
         }
-        const int ci = q >> 5, lane = q & 31;
-        if constexpr (MIXED) {
-            constexpr int NC = PredMx<ORDER>::ncomp;
-            float *c = static_cast<float *>(out) + ci * NC * 32 + lane;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const float hi = __double2float_rn(x[k]);
-                c[(PMX_XH + k) * 32] = hi;
-                c[(PMX_XL + k) * 32] = __double2float_rn(x[k] - (double)hi);
-                c[(PMX_V + k) * 32] = __double2float_rn(v[k]);
-                if constexpr (ORDER >= 6) c[(PMX_A + k) * 32] = __double2float_rn(a[k]);
-                if constexpr (ORDER == 8) c[(PMX_J + k) * 32] = __double2float_rn(jk[k]);
-            }
-            c[PMX_M * 32] = __double2float_rn(m);
-        } else {
-            constexpr int NC = Pred64<ORDER>::ncomp;
-            double *c = static_cast<double *>(out) + ci * NC * 32 + lane;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                c[(P64_X + k) * 32] = x[k];
-                c[(P64_V + k) * 32] = v[k];
-                if constexpr (ORDER >= 6) c[(P64_A + k) * 32] = a[k];
-                if constexpr (ORDER >= 8) c[(P64_J + k) * 32] = jk[k];
-                if constexpr (ORDER == 9) c[(P64_XL + k) * 32] = xl[k];
-            }
-            c[P64_M * 32] = m;
-        }
+        unsigned char *chunk = static_cast<unsigned char *>(out) + (q >> 5) * Layout<ORDER, MIXED>::chunk_bytes;
+        put_predicted<ORDER, MIXED>(chunk + (q & 31) * (MIXED ? 4 : 8), x, v, a, jk, xl, m);
     }
 }
 

@@ -71,11 +71,10 @@ struct IntStatus {
 };
 
 struct Sched {
-    unsigned long long tnext_bits;   // min(tlast + dt) as the bits of a positive double
-    int nact;                        // active slots of the current step
-    int work;                        // next force work item
+    unsigned long long next_bits;    // min(tlast + dt) as the bits of a positive double
+    int nact[2];                     // active slots, of even and odd steps in turn
+    int work;                        // force work items taken beyond the first per CTA
     int error;                       // 1: a timestep underflowed, 2: a device wait gave up
-    int pad;
     double tnext, dtlim, tsys, tend;
     double eps2, etapow, dtmax;
     long long particle_steps, block_steps;
@@ -90,26 +89,29 @@ double recalc_dt(int order, const double *rec, const double *aux, double eta, do
 struct IntegratorLaunch {
     double *jp;          // records (the state)
     double *dt;          // per-slot timestep
+    double *tn;          // per-slot tlast + dt, kept from integrator_start on
     double *aux;         // per-slot dump derivatives [kAuxWords]
+    void *pred;          // predicted slots
     int *ilist;          // active slots
     Sched *sched;
     double *force, *partial;
-    unsigned *counter;
     int *err;
     int n, nchunk, nsm;
     size_t partial_cap;
-    int target_items, items_grid, smem_fp64, smem_mixed;
-    int big_grid;       // grid of the large-step force kernel
     bool mixed;
 };
 
-cudaError_t integrator_step_launch(int order, const IntegratorLaunch &L, cudaStream_t s);
+// Before a run: tlast + dt per slot, the first block time, counters.
+cudaError_t integrator_start(int order, const IntegratorLaunch &L, cudaStream_t s);
+// One block step; par alternates between 0 and 1, starting with 0 after
+// integrator_start.
+cudaError_t integrator_step_launch(int order, const IntegratorLaunch &L, int par, cudaStream_t s);
 
 // Persistent engine (hb_integrator.cu): one cooperative launch runs up to
-// max_steps block steps; gbar is two zeroed words (grid barrier); spin is the
-// poll limit of a barrier wait.  setup: dynamic shared memory and resident
-// CTAs per SM of the kernel.
-cudaError_t persistent_setup(int order, bool mixed, int *smem, int *per_sm);
+// max_steps block steps (an even number, except the last launch before an
+// integrator_start); gbar is two zeroed words (grid barrier); spin is the
+// poll limit of a barrier wait.  setup: resident CTAs per SM of the kernel.
+cudaError_t persistent_setup(int order, bool mixed, int *per_sm);
 cudaError_t persistent_launch(int order, const IntegratorLaunch &L, unsigned *gbar,
                               long long max_steps, unsigned spin, int grid, cudaStream_t s);
 
@@ -155,8 +157,7 @@ int team_shape(int order, const TeamConfig &cfg, int nmax, TeamLaunch *L);
 cudaError_t team_launch(int order, const TeamLaunch &L, int teams, cudaStream_t s);
 cudaError_t team_sched_sync(Sched *s, TeamState *st, bool to_team, cudaStream_t stream);
 
-cudaError_t integrator_kernel_setup(int order, bool mixed, int *smem, int *blocks_per_sm,
-                                    int *big_per_sm);
+cudaError_t integrator_kernel_setup(int order, bool mixed);
 cudaError_t integrator_assign(int order, double *jp, double *dt, const double *force, int n,
                               int set_dt, double eta_s, double dtmax, cudaStream_t s);
 cudaError_t integrator_energy(int order, const double *jp, const double *pot, int n, double *part,

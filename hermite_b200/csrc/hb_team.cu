@@ -79,23 +79,6 @@ __device__ __forceinline__ double warp_min(double v)
     return v;
 }
 
-// calc_dtlim (SRC/nbodysystem.h:652-661): dtmax halved until tnext is a
-// multiple of it, at most 64 times.  For a power-of-two dtmax = 2^D this is
-// 2^(D-k) with k = clamp(D - e, 0, 64), e the exponent of the lowest set
-// bit of tnext (tnext = 0 is a multiple of everything): the same value the
-// reference's loop reaches, from the exponent and significand bits.
-__device__ __forceinline__ double team_dtlim(double tnext, double dtmax)
-{
-    if (!(tnext > 0.0)) return dtmax;
-    const long long b = __double_as_longlong(tnext);
-    const int ex = (int)((b >> 52) & 0x7ff);
-    const long long sig = (b & 0xfffffffffffffll) | (ex ? (1ll << 52) : 0ll);
-    const int e = (ex ? ex : 1) - 1075 + (__ffsll(sig) - 1);
-    const int D = (int)((__double_as_longlong(dtmax) >> 52) & 0x7ff) - 1023;
-    const int k = max(0, min(64, D - e));
-    return __longlong_as_double(__double_as_longlong(dtmax) - ((long long)k << 52));
-}
-
 // Partial forces of nr i-particles (ibuf, AoSoA32, at positions idx(gi))
 // against this CTA's JL own predicted slots.  G lanes (a power of two)
 // share NI i-particles, each lane summing every G-th own slot, and their
@@ -305,7 +288,7 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
             const int kact = __shfl_sync(0xffffffffu, kk, rank);
             const int myoff = __shfl_sync(0xffffffffu, incl, rank) - kact;
             if (dead || err || !(tnext <= L.tend) || steps >= L.max_steps) break;
-            const double dtlim = team_dtlim(tnext, L.dtmax);
+            const double dtlim = calc_dtlim(tnext, L.dtmax);
             if (w == 0) {
                 koff[lane + 1] = incl;
                 if (lane == 0) koff[0] = 0;
@@ -559,7 +542,6 @@ __global__ void team_to_sched_kernel(const TeamState *st, Sched *s)
     s->particle_steps = st->particle_steps;
     s->block_steps = st->block_steps;
     if (st->error) s->error = st->error;
-    s->tnext_bits = 0x7ff0000000000000ull;
     IntStatus *o = s->status;
     o->tsys = s->tsys;
     o->particle_steps = s->particle_steps;

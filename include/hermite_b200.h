@@ -188,7 +188,7 @@ int hb_force_variant_info(int order, int precision, int variant,
 int hb_integrator_init(hb_ctx *ctx, double tsys, double eps2, double eta, double eta_s,
                        double dtmax);
 /* Engines for hb_integrator_run (same state, same algorithm):
- *  HB_ENGINE_GRAPH  four phases (five kernels) per block step over the whole GPU, 32 steps
+ *  HB_ENGINE_GRAPH  three kernels per block step over the whole GPU, 32 steps
  *                   per replay of a CUDA graph (any N, FP64 or mixed);
  *  HB_ENGINE_PERSISTENT  the graph engine's phases in one cooperative kernel
  *                   whose CTAs all stay resident, grid barriers (bounded
@@ -199,7 +199,7 @@ int hb_integrator_init(hb_ctx *ctx, double tsys, double eps2, double eta, double
  *                   block-step loop in one kernel, three cluster barriers per
  *                   step (FP64; N up to 16 x the slots one CTA holds in
  *                   shared memory, about 16k);
- *  HB_ENGINE_AUTO   the team engine for FP64 systems of up to 3072
+ *  HB_ENGINE_AUTO   the team engine for FP64 systems of up to 2560
  *                   particles, else the graph engine (the default).
  * team_ctas: CTAs per team (1..16), 0 = chosen from N. */
 enum { HB_ENGINE_AUTO = 0, HB_ENGINE_GRAPH = 1, HB_ENGINE_TEAM = 2, HB_ENGINE_PERSISTENT = 3 };
