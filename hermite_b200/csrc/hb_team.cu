@@ -8,20 +8,27 @@
 // when each step is its own set of kernels; for N of a few thousand the
 // force itself is smaller than that.  Here C CTAs of one cluster own the
 // system's slots in C contiguous 32-slot-aligned ranges and run every step
-// with three cluster barriers and no grid-wide synchronisation:
+// with two cluster barriers and no grid-wide synchronisation:
 //
-//   A  each CTA: minimum of tlast + dt over its own slots       -> barrier 1
-//   B  every CTA reads the C minima (distributed shared memory): tnext;
-//      each CTA lists its own active slots (slot order) and predicts its own
-//      slots to tnext into shared memory                        -> barrier 2
-//   C  every CTA gathers the predicted states of all active slots from
-//      their owners and sums them against its own slots (a j-split across
-//      the team), partial forces in its shared memory           -> barrier 3
-//      each owner adds the C partials of its active slots in rank order and
+//   A  each CTA: minimum of tlast + dt over its own slots, and the slots at
+//      it; their states, predicted to it, pushed with the minimum into every
+//      CTA (distributed shared memory), one warp per receiver  -> barrier 1
+//   B  every CTA: tnext, the minimum of the minima; its own slots predicted to
+//      tnext; the active states summed against them (a j-split across the
+//      team), each partial force pushed to the state's owner    -> barrier 3
+//   C  each owner adds the C partials of its active slots in rank order and
 //      runs the corrector (Particle::correct + the quantised Aarseth step)
 //
 // Steps with more active slots than the push regions hold are processed in
-// rounds pulled from the owners.
+// rounds pulled from the owners, behind one more barrier (2); the regions hold
+// every slot where the shared memory allows it.
+//
+// What bounds a step at N = 1024 (16 CTAs, 6.6 us, from 8.2 us with one warp
+// pushing to all ranks, minima by shuffles and 6 % of the steps in rounds): the
+// partial forces, a chain of FP64 latencies over a few j per lane, about 2 us;
+// the two barriers with the pushes behind them, 2 us; the corrector and the
+// candidates 1 us; the prediction and the prefix sums 0.6 us.  Unrolling the j
+// loop by 4 or 8 instead of 2 measured 0.4 us slower.
 // Teams take systems from a device counter, so one launch integrates a whole
 // ensemble with every system on its own block-time sequence (no lockstep),
 // or a single system.  The per-system state is the same record array and dt
@@ -73,17 +80,24 @@ struct TeamSmem {
 // Smallest round with the records in global memory (larger systems).
 constexpr int kTeamIMinGlobal = 64;
 
+// Minimum over the warp of positive doubles (block times; +inf for none), whose
+// bit patterns order like the values: the high words' minimum, then the low
+// words' among the lanes that have it.  Two warp reductions, a quarter of the
+// time of five shuffles and compares of doubles.
 __device__ __forceinline__ double warp_min(double v)
 {
-    for (int o = 16; o; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const unsigned hi = (unsigned)(b >> 32);
+    const unsigned mh = __reduce_min_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_min_sync(0xffffffffu, hi == mh ? (unsigned)b : 0xffffffffu);
+    return __longlong_as_double((long long)(((unsigned long long)mh << 32) | ml));
 }
 
 // Partial forces of nr i-particles (ibuf, AoSoA32, at positions idx(gi))
 // against this CTA's JL own predicted slots.  G lanes (a power of two)
 // share NI i-particles, each lane summing every G-th own slot, and their
-// sums meet in a fixed xor-shuffle tree; out(gi, f) is called by the first
-// lane of each group.  NW * 32 / G * NI >= nr i-slots.
+// sums meet in a fixed xor-shuffle tree; out(idx, f) is called by the first
+// lane of each group.
 template <int ORDER, int NI, typename Idx, typename Out>
 __device__ __forceinline__ void team_force_ni(const double *ibuf, const double *pred, int JL, int nr,
                                               double eps2, Idx idx, Out out)
@@ -92,36 +106,41 @@ __device__ __forceinline__ void team_force_ni(const double *ibuf, const double *
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int G = 32;
     while (G > 1 && NW * (32 / G) * NI < nr) G >>= 1;
-    const int gp = w * (32 / G) + lane / G, js = lane & (G - 1);
-    double f[NI][F];
+    const int js = lane & (G - 1), slots = NW * (32 / G);
+    // more than a pair of i per thread: in rounds
+    for (int g0 = 0; g0 * NI < nr; g0 += slots) {
+        const int gp = g0 + w * (32 / G) + lane / G;
+        double f[NI][F];
 #pragma unroll
-    for (int n = 0; n < NI; ++n)
+        for (int n = 0; n < NI; ++n)
 #pragma unroll
-        for (int c = 0; c < F; ++c) f[n][c] = 0.0;
-    if (gp * NI < nr) {
-        Body64 I[NI];
+            for (int c = 0; c < F; ++c) f[n][c] = 0.0;
+        int x[NI];
+        if (gp * NI < nr) {
+            Body64 I[NI];
 #pragma unroll
-        for (int n = 0; n < NI; ++n) {
-            const int x = idx(gp * NI + n < nr ? gp * NI + n : gp * NI);   // a missing pair partner repeats the first
-            load_i64<ORDER>(ibuf, x >> 5, x & 31, I[n]);
-        }
+            for (int n = 0; n < NI; ++n) {
+                x[n] = idx(gp * NI + n < nr ? gp * NI + n : gp * NI);   // a missing pair partner repeats the first
+                load_i64<ORDER>(ibuf, x[n] >> 5, x[n] & 31, I[n]);
+            }
 #pragma unroll 2
-        for (int j = js; j < JL; j += G) {
-            Body64 J;
-            load_i64<ORDER>(pred, j >> 5, j & 31, J);
+            for (int j = js; j < JL; j += G) {
+                Body64 J;
+                load_i64<ORDER>(pred, j >> 5, j & 31, J);
 #pragma unroll
-            for (int n = 0; n < NI; ++n) interact64<ORDER>(I[n], J, eps2, f[n]);
+                for (int n = 0; n < NI; ++n) interact64<ORDER>(I[n], J, eps2, f[n]);
+            }
         }
+        for (int o = G >> 1; o; o >>= 1)
+#pragma unroll
+            for (int n = 0; n < NI; ++n)
+#pragma unroll
+                for (int c = 0; c < F; ++c) f[n][c] += __shfl_xor_sync(0xffffffffu, f[n][c], o);
+        if (js == 0)
+#pragma unroll
+            for (int n = 0; n < NI; ++n)
+                if (gp * NI + n < nr) out(x[n], f[n]);
     }
-    for (int o = G >> 1; o; o >>= 1)
-#pragma unroll
-        for (int n = 0; n < NI; ++n)
-#pragma unroll
-            for (int c = 0; c < F; ++c) f[n][c] += __shfl_xor_sync(0xffffffffu, f[n][c], o);
-    if (js == 0)
-#pragma unroll
-        for (int n = 0; n < NI; ++n)
-            if (gp * NI + n < nr) out(gp * NI + n, f[n]);
 }
 
 // Two i per lane (two independent chains per j load) at 4th order, where the
@@ -150,7 +169,7 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
     const int C = (int)team.num_blocks(), rank = (int)team.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int jl_cap = L.jl_cap;   // own slots per CTA
-    const int IM = L.im;           // i states per round (<= NW * 32)
+    const int IM = L.im;           // i states per round
     const int KM = IM / C;         // i states one rank pushes per step (its region of ibuf)
 
     extern __shared__ __align__(16) unsigned char smem[];
@@ -166,6 +185,8 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
     int *gc = gq + IM;                                            // [IM]
     int *koff = gc + IM;                                          // [48] koff[c] = actives below rank c
     int *misc = koff + 48;                                        // [0] system (rank 0), [1] own error
+    __shared__ TeamXch own_xch;                                   // this rank's (m, k, err)
+    TeamXch *own = &own_xch;
 
     const double inf = __longlong_as_double(0x7ff0000000000000ll);
 
@@ -212,10 +233,12 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
         int err = 0;
         __syncthreads();
 
-        // Warp 0, before every barrier 1: the own minimum, its candidates (in
-        // slot order), their states predicted to it pushed into region `rank`
-        // of every CTA's ibuf, and (m, k, err) into every CTA's xa[rank].
-        auto announce = [&]() {
+        // Before every barrier 1.  Warp 0: the own minimum and its candidates (in
+        // slot order).  Then every warp c < C pushes to rank c: the candidates'
+        // states predicted to the minimum into region `rank` of its ibuf, one
+        // per lane, and (m, k, err) into its xa[rank].  (One warp pushing to all
+        // ranks in turn took 0.4 us longer at 16 ranks.)
+        auto find_candidates = [&]() {
             double m = inf;
             for (int q = lane; q < JL; q += 32) m = fmin(m, tn[q]);
             m = warp_min(m);
@@ -229,40 +252,40 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
                     k += __popc(b);
                 }
             }
-            __syncwarp();
-            // the candidates' states predicted to m, pushed by one lane each
-            // into region `rank` of every CTA's ibuf (store instructions of
-            // one lane go to one rank back to back, from registers)
-            const int kp = min(k, KM);
-            for (int a = lane; a < kp; a += 32) {
-                const double *r = rec + (size_t)cand[a] * R;
-                double x[3], v[3], ac[3] = {0.0, 0.0, 0.0}, jk[3] = {0.0, 0.0, 0.0};
-                double xl[3] = {0.0, 0.0, 0.0};
-                predict_slot<ORDER>(r, m, x, v, ac, jk, xl);
-                const double mass = r[3];
-                const int g = rank * KM + a;
-                const int off = (g >> 5) * P * 32 + (g & 31);
-                for (int c = 0; c < C; ++c) {
-                    double *d = team.map_shared_rank(ibuf, c) + off;
-#pragma unroll
-                    for (int kk = 0; kk < 3; ++kk) {
-                        d[(P64_X + kk) * 32] = x[kk];
-                        d[(P64_V + kk) * 32] = v[kk];
-                        if constexpr (ORDER >= 6) d[(P64_A + kk) * 32] = ac[kk];
-                        if constexpr (ORDER >= 8) d[(P64_J + kk) * 32] = jk[kk];
-                        if constexpr (ORDER == 9) d[(P64_XL + kk) * 32] = xl[kk];
-                    }
-                    d[P64_M * 32] = mass;
-                }
-            }
-            if (lane < C) {
-                TeamXch *d = team.map_shared_rank(xa, lane) + rank;
-                d->m = m;
-                d->k = k;
-                d->err = misc[1];
+            if (lane == 0) {
+                own->m = m;
+                own->k = k;
+                own->err = misc[1];
             }
         };
-        if (w == 0) announce();
+        auto announce = [&]() {
+            if (w >= C) return;
+            const TeamXch x = *own;
+            const int kp = min(x.k, KM);
+            double *to = team.map_shared_rank(ibuf, w);
+            for (int a = lane; a < kp; a += 32) {
+                const double *r = rec + (size_t)cand[a] * R;
+                double p[3], v[3], ac[3] = {0.0, 0.0, 0.0}, jk[3] = {0.0, 0.0, 0.0};
+                double xl[3] = {0.0, 0.0, 0.0};
+                predict_slot<ORDER>(r, x.m, p, v, ac, jk, xl);
+                const double mass = r[3];
+                const int g = rank * KM + a;
+                double *d = to + (g >> 5) * P * 32 + (g & 31);
+#pragma unroll
+                for (int kk = 0; kk < 3; ++kk) {
+                    d[(P64_X + kk) * 32] = p[kk];
+                    d[(P64_V + kk) * 32] = v[kk];
+                    if constexpr (ORDER >= 6) d[(P64_A + kk) * 32] = ac[kk];
+                    if constexpr (ORDER >= 8) d[(P64_J + kk) * 32] = jk[kk];
+                    if constexpr (ORDER == 9) d[(P64_XL + kk) * 32] = xl[kk];
+                }
+                d[P64_M * 32] = mass;
+            }
+            if (lane == 0) team.map_shared_rank(xa, w)[rank] = x;
+        };
+        if (w == 0) find_candidates();
+        __syncthreads();
+        announce();
 
         for (;;) {
             team.sync();   // barrier 1: every rank's (m, k, err) and pushed states are here
@@ -322,33 +345,40 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
             __syncthreads();
 
             if (!over && nact <= IM) {
-                // the active states are the pushed ones: position gi of rank c
+                // the active states are the pushed ones: active a of rank c
                 // sits at ibuf[c * KM + a]; partials go to the owner's part
                 // at [rank * KM + a]
                 team_force<ORDER>(
                     ibuf, pred, JL, nact, eps2,
                     [&](int gi) {
+                        // koff is ascending: the last rank with koff[c] <= gi
                         int c = 0;
-                        while (c + 1 < C && gi >= koff[c + 1]) ++c;
+#pragma unroll
+                        for (int step = 8; step; step >>= 1)
+                            if (c + step < C && koff[c + step] <= gi) c += step;
                         return c * KM + (gi - koff[c]);
                     },
-                    [&](int gi, const double *f) {
-                        int c = 0;
-                        while (c + 1 < C && gi >= koff[c + 1]) ++c;
-                        double *d = team.map_shared_rank(part, c) + (size_t)(rank * KM + gi - koff[c]) * F;
+                    [&](int x, const double *f) {
+                        const int c = x / KM;
+                        double *d = team.map_shared_rank(part, c) + (size_t)(rank * KM + x - c * KM) * F;
 #pragma unroll
                         for (int k = 0; k < F; ++k) d[k] = f[k];
                     });
                 team.sync();   // barrier 3: every partial is with its owner
 
                 if (w == 0) {
+                    // the ranks' partials in rank order, one value per lane
+                    for (int e = lane; e < kact * F; e += 32) {
+                        double v = part[e];
+#pragma unroll 4
+                        for (int src = 1; src < C; ++src) v += part[(size_t)src * KM * F + e];
+                        part[e] = v;
+                    }
+                    __syncwarp();
                     for (int a = lane; a < kact; a += 32) {
                         double f[F];
 #pragma unroll
-                        for (int k = 0; k < F; ++k) f[k] = 0.0;
-                        for (int src = 0; src < C; ++src)
-#pragma unroll
-                            for (int k = 0; k < F; ++k) f[k] += part[(size_t)(src * KM + a) * F + k];
+                        for (int k = 0; k < F; ++k) f[k] = part[a * F + k];
                         const int q = cand[a];
                         double *r = rec + (size_t)q * R;
                         const double dtn = correct_particle<ORDER>(
@@ -359,8 +389,10 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
                         tn[q] = dtn + r[7];
                     }
                     __syncwarp();
-                    announce();
+                    find_candidates();
                 }
+                __syncthreads();
+                announce();
             } else {
                 // many actives: rounds of IM pulled from the owners
                 team.sync();   // barrier 2: predicted states and candidate lists complete
@@ -411,7 +443,9 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
                     if (base + IM < nact) team.sync();   // part and ibuf are reused by the next round
                 }
                 __syncthreads();
-                if (w == 0) announce();
+                if (w == 0) find_candidates();
+                __syncthreads();
+                announce();
             }
             ++steps;
             psteps += nact;
@@ -484,8 +518,8 @@ cudaError_t team_setup_t(int ctas, TeamConfig *cfg)
 }
 
 // Launch shape for systems of up to nmax particles: the own slots per CTA
-// they need, and as many i-states per round (a multiple of 32, at most one
-// per thread) as the rest of the shared memory holds.
+// they need, and as many i-states per round (a multiple of 32, at most the
+// system's slots) as the rest of the shared memory holds.
 template <int ORDER>
 int team_shape_t(const TeamConfig &cfg, int nmax, TeamLaunch *L)
 {
@@ -496,7 +530,10 @@ int team_shape_t(const TeamConfig &cfg, int nmax, TeamLaunch *L)
     if (!rsmem && jl > cfg.jl_cap_g) return -1;
     long long im = ((long long)cfg.smem - (long long)SM::fixed - (long long)SM::per_slot(rsmem) * jl) /
                    (long long)SM::per_i;
-    im = std::min<long long>(im & ~31LL, kTeamWarps * 32);
+    // every slot of the team where that fits, so that no step overflows the
+    // push regions: at N = 1024, 4th order, 6 % of the steps did with 512 and took
+    // 33 us each in the pull path, 2 us of the mean step
+    im = std::min<long long>(im & ~31LL, std::max((long long)kTeamWarps * 32, (long long)jl * cfg.ctas));
     if (im < (rsmem ? kTeamIMax : kTeamIMinGlobal)) return -1;
     L->ctas = cfg.ctas;
     L->jl_cap = jl;
