@@ -283,10 +283,10 @@ potential_kernel(const double *__restrict__ posm, int nchunk, int n, double eps2
 //
 // Groups of 1024 slots (8 warps x 4 chunks of i-particles, one per lane and
 // chunk) meet every later chunk: lane l of a warp takes j = l + s of the chunk
-// in step s, the chunk's states and its running sums moving one lane per step
-// by shuffles (10 shuffles for 4 pairs, against 52 FP64 instructions).  So a
-// step adds to 4 i-sums and to one j-sum of every lane with no collisions, and
-// after 32 steps the j-sums are home.  The 8 warps' j-sums meet in shared
+// in step s, the chunk's running sums moving one lane per step by a shuffle
+// (the states moving along instead of being read again measured 4 % slower).
+// So a step adds to 4 i-sums and to one j-sum of every lane with no collisions,
+// and after 32 steps the j-sums are home.  The 8 warps' j-sums meet in shared
 // memory and go out once per (group, j).  The group's own chunks are summed
 // one-sided, as ordered pairs; the self pair is step 0 of a chunk with itself.
 //
@@ -294,8 +294,8 @@ potential_kernel(const double *__restrict__ posm, int nchunk, int n, double eps2
 // slices of `lc` chunks; pot_band_kernel then adds rows and slices to the
 // potentials in a fixed order, so results are deterministic.
 //
-// N = 100003: 5.27 ms (11.0 ms with ordered pairs and no slices), 65 % of the
-// FP64 pipe's rate on the 13 instructions per pair; 8 i-chunks a warp, 2 of
+// N = 100003: 5.08 ms (11.0 ms with ordered pairs and no slices); the FP64 pipe
+// is 80 % busy, its 13 instructions per pair and little else; 8 i-chunks a warp, 2 of
 // 16 warps, three CTAs per SM and other unrollings measured 0-10 % slower.
 constexpr int kSymWarps = 8, kSymI = 4, kSymTile = 16;
 constexpr int kSymChunks = kSymWarps * kSymI, kSymSlots = kSymChunks * 32;
@@ -318,14 +318,15 @@ __device__ __forceinline__ void pot_chunk(const double *cp, int lane, const doub
                                           const double (&mi)[kSymI], const bool (&own)[kSymI],
                                           double eps2, double (&total)[kSymI], double &fj)
 {
-    double x = cp[lane], y = cp[32 + lane], z = cp[64 + lane], m = cp[96 + lane];
     double part[kSymI];
 #pragma unroll
     for (int k = 0; k < kSymI; ++k) part[k] = 0.0;
     fj = 0.0;
     const int next = (lane + 1) & 31;
+    int jl = lane;
 #pragma unroll 4
     for (int s = 0; s < 32; ++s) {
+        const double x = cp[jl], y = cp[32 + jl], z = cp[64 + jl], m = cp[96 + jl];
 #pragma unroll
         for (int k = 0; k < kSymI; ++k) {
             const double dx = x - xi[k][0], dy = y - xi[k][1], dz = z - xi[k][2];
@@ -334,10 +335,7 @@ __device__ __forceinline__ void pot_chunk(const double *cp, int lane, const doub
             part[k] = fma(-m, ri, part[k]);
             if (!DIAG) fj = fma(-mi[k], ri, fj);
         }
-        x = __shfl_sync(0xffffffffu, x, next);
-        y = __shfl_sync(0xffffffffu, y, next);
-        z = __shfl_sync(0xffffffffu, z, next);
-        m = __shfl_sync(0xffffffffu, m, next);
+        jl = (jl + 1) & 31;
         if (!DIAG) fj = __shfl_sync(0xffffffffu, fj, next);
     }
 #pragma unroll
@@ -493,7 +491,7 @@ static cudaError_t launch_potential_sym(int n, int npad, double eps2, const doub
 }
 
 // From this many slots on the pairs are taken once: 16384: 191 against 283 us
-// with ordered pairs, 100003: 5.27 against 8.90 ms, 262144: 34.3 against 60.8;
+// with ordered pairs, 100003: 5.08 against 8.90 ms, 262144: 34.3 against 60.8;
 // 12000: 189 against 171 us, too few groups to fill the GPU evenly.
 // Double-double positions keep the ordered pairs.
 constexpr int kPotSymMin = 14336;
