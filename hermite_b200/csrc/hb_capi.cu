@@ -317,6 +317,29 @@ int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
         return HB_OK;
     }
     const bool automatic = ctx->variant_override < 0 && ctx->jsplit_override == 0;
+    if (automatic && force_out_dev == ctx->d_force &&
+        force_sym_takes(ctx->order, mixed, nact, ctx->npad, ctx->partial_cap)) {
+        // most particles move: every pair once
+        if (ctx->pred_stale) {
+            HB_CK(launch_predict(ctx->order, mixed, ctx->d_jp, ctx->nbody, ctx->npad, ctx->tsys,
+                                 ctx->d_pred, ctx->d_err, ctx->stream));
+            ctx->launches++;
+            ctx->pred_stale = false;
+        }
+        ForceArgs a{};
+        a.pred = ctx->d_pred;
+        a.nchunk = ctx->npad / 32;
+        a.nact = nact;
+        a.eps2 = eps2;
+        a.force = force_out_dev;
+        a.partial = ctx->d_partial;
+        a.err = ctx->d_err;
+        a.spin = ctx->wait_limit;
+        int launches = 0;
+        HB_CK(launch_force_sym(ctx->order, a, ctx->partial_cap, ctx->nsm, ctx->stream, &launches));
+        ctx->launches += launches;
+        return HB_OK;
+    }
     int jsplit_hint = 0;
     const int v = automatic ? auto_variant(ctx, nact) : pick_variant(ctx, nact, &jsplit_hint);
     const ForceVariant *fv = force_variant(ctx->order, mixed, v);
@@ -489,7 +512,10 @@ int hb_create(int order, int nbody, int precision, hb_ctx **out)
     const size_t np = ctx->npad;
     const size_t pred_bytes = std::max(np * pred64_ncomp(order) * sizeof(double),
                                        np * predmx_ncomp(order) * sizeof(float));
-    ctx->partial_cap = (size_t)2 * ctx->nsm * 8 * 256 * ctx->F;
+    // j-slices' partials; or rows of one double per value and slot for pairs
+    // taken once, 16 rows up to 256 MiB
+    ctx->partial_cap = std::max((size_t)2 * ctx->nsm * 8 * 256 * ctx->F,
+                                std::min(16 * np * ctx->F, (size_t)32 << 20));
     bool ok = true;
     ok = ok && cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&ctx->ev_upload, cudaEventDisableTiming) == cudaSuccess;

@@ -1,0 +1,75 @@
+// hb_force_sym.cu -- launches of the each-pair-once FP64 force.
+#include <algorithm>
+
+#include "hb_force_sym.cuh"
+
+namespace hb {
+namespace {
+
+template <int ORDER>
+cudaError_t launch_t(const ForceArgs &f, size_t cap, int nsm, cudaStream_t s, int *launches)
+{
+    constexpr int F = Frc<ORDER>::words, GC = SymShape<ORDER>::GC;
+    cudaError_t e = cudaFuncSetAttribute(force_sym_kernel<ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         SymShape<ORDER>::bytes);
+    if (e != cudaSuccess) return e;
+    SymArgs a{};
+    a.pred = static_cast<const double *>(f.pred);
+    a.force = f.force;
+    a.nchunk = f.nchunk;
+    a.nact = f.nact;
+    a.ca = (f.nact + 31) / 32;
+    a.eps2 = f.eps2;
+    a.err = f.err;
+    a.spin = f.spin;
+    const int groups = (a.ca + GC - 1) / GC;
+    const long long chunk = F * 32, room = (long long)(cap / chunk);   // scratch in [F][32] blocks
+    for (int g0 = 0; g0 < groups; g0 += a.ng) {
+        // about 6 waves of CTAs: a CTA's chunks, in whole tiles (3 and 12 waves
+        // measured 2-5 % slower)
+        const long long wide = std::max(1LL, std::min((long long)groups - g0, room / a.ca));
+        const long long units = wide * (a.nchunk - (long long)g0 * GC);
+        const long long lc = units / (6LL * SymShape<ORDER>::MINB * nsm);
+        a.g0 = g0;
+        a.lc = (int)std::max(1LL, (lc + kSymFTile - 1) / kSymFTile) * kSymFTile;
+        a.smax = sym_slices(a.nchunk, g0, GC, a.lc);
+        a.ng = (int)std::min((long long)(groups - g0), room / (a.ca + (long long)a.smax * GC));
+        if (a.ng < 1) return cudaErrorInvalidValue;
+        a.rows = f.partial;
+        a.cols = f.partial + (size_t)a.ng * a.ca * chunk;
+        int ctas = 0;
+        for (int g = g0; g < g0 + a.ng; ++g) ctas += sym_slices(a.nchunk, g, GC, a.lc);
+        e = launch_pdl(force_sym_kernel<ORDER>, dim3(ctas), kSymFWarps * 32, SymShape<ORDER>::bytes, s, a);
+        const long long values = (long long)(a.ca - g0 * GC) * chunk;
+        if (e == cudaSuccess)
+            e = launch_pdl(sym_band_kernel<ORDER>, dim3((unsigned)((values + 255) / 256)), 256, 0, s, a);
+        if (e != cudaSuccess) return e;
+        *launches += 2;
+    }
+    return cudaSuccess;
+}
+
+}  // namespace
+
+// Both sides measured (ms, ordered pairs / pairs once): all of N = 4096 0.060 /
+// 0.049 at 4th order and 0.088 / 0.090 at 6th, 12000 0.526 / 0.425 (6th), 131072
+// 59.9 / 41.4 (6th); parts of N = 131072 at 6th order: 20000 8.93 / 8.94,
+// 45000 20.0 / 19.2, 70000 31.3 / 27.5; of 65536 at 4th: 20000 2.61 / 2.69, 30000
+// 3.90 / 3.69.  The 8th-order sums are compensated; they keep ordered pairs.
+bool force_sym_takes(int order, bool mixed, int nact, int npad, size_t cap)
+{
+    if (mixed || (order != 4 && order != 6)) return false;
+    const size_t blocks = cap / (size_t)(3 * (order / 2) * 32);
+    return nact >= 4096 && nact >= npad * 4LL / 10 && blocks >= (size_t)npad / 32 * 2;
+}
+
+cudaError_t launch_force_sym(int order, const ForceArgs &f, size_t cap, int nsm, cudaStream_t s, int *launches)
+{
+    switch (order) {
+    case 4: return launch_t<4>(f, cap, nsm, s, launches);
+    case 6: return launch_t<6>(f, cap, nsm, s, launches);
+    }
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace hb

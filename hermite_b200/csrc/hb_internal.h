@@ -174,6 +174,11 @@ const ForceVariant *force_variant(int order, bool mixed, int v);
 constexpr int kLanesMaxAct = 16;
 cudaError_t launch_force_lanes(int order, const ForceArgs &a, int nsm, cudaStream_t s, int *launches);
 
+// FP64 force with every pair of active particles taken once (hb_force_sym.cuh);
+// needs f.pred and f.partial (cap doubles); *launches is advanced.
+bool force_sym_takes(int order, bool mixed, int nact, int npad, size_t cap);
+cudaError_t launch_force_sym(int order, const ForceArgs &f, size_t cap, int nsm, cudaStream_t s,
+                             int *launches);
 cudaError_t launch_predict(int order, bool mixed, const double *jp, int n, int npad,
                            double tsys, void *pred, int *err, cudaStream_t s);
 // Potential of n slots; partial: scratch of cap doubles; *launches is advanced.
