@@ -101,6 +101,18 @@ __device__ __forceinline__ int ens_split(int cnt, int npad)
     return max(1, min(kEnsSplit / tiles, npad / 128));
 }
 
+// Initial conditions: tlast = tsys and derivatives zero for every real slot.
+__global__ void __launch_bounds__(kClusterPad)
+ens_reset_kernel(double *jp, int R, const Cluster *cl, const int *slot_cluster, double tsys)
+{
+    const int slot = blockIdx.x * kClusterPad + threadIdx.x;
+    const Cluster c = cl[slot_cluster[blockIdx.x]];
+    if (slot - c.off >= c.n) return;
+    double *r = jp + (size_t)slot * R;
+    r[7] = tsys;
+    for (int k = 8; k < R; ++k) r[k] = 0.0;
+}
+
 // 1. next block time; reset the per-cluster counters
 template <int ORDER>
 __global__ void ens_min_kernel(EnsLaunch L)
@@ -1068,6 +1080,33 @@ int hb_ens_get_cluster(hb_ens *e, int c, double *records, double *dt)
     return ce == cudaSuccess ? HB_OK : ens_fail(e, HB_ERR_CUDA, "hb_ens_get_cluster", ce);
 }
 
+}  // extern "C"
+
+namespace {
+// The lockstep engine's captured steps, made by the first run that needs them
+// (the team engine does not: 0.7 ms of each start-up).
+int ensure_graph(hb_ens *e)
+{
+    if (e->exec) return HB_OK;
+    cudaError_t ce = cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal);
+    if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "capture", ce);
+    cudaError_t le = cudaSuccess;
+    for (int k = 0; k < kEnsStepsPerGraph && le == cudaSuccess; ++k) le = dispatch_step(e);
+    cudaGraph_t g = nullptr;
+    ce = cudaStreamEndCapture(e->stream, &g);
+    if (le != cudaSuccess || ce != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        return ens_fail(e, HB_ERR_CUDA, "capturing the ensemble step graph",
+                        le != cudaSuccess ? le : ce);
+    }
+    e->graph = g;
+    ce = cudaGraphInstantiate(&e->exec, g, 0);
+    if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "instantiate", ce);
+    return HB_OK;
+}
+}  // namespace
+
+extern "C" {
 int hb_ens_init(hb_ens *e, double tsys, double eta, double eta_s, double dtmax)
 {
     if (!e) return HB_ERR_INVALID;
@@ -1079,25 +1118,13 @@ int hb_ens_init(hb_ens *e, double tsys, double eta, double eta_s, double dtmax)
     if (e->exec) { cudaGraphExecDestroy(e->exec); e->exec = nullptr; }
     if (e->graph) { cudaGraphDestroy(e->graph); e->graph = nullptr; }
     e->ready = false;
-    // tlast = tsys, derivatives zero, for every real slot (device copy)
-    std::vector<double> rec;
-    for (int c = 0; c < e->nclusters; ++c) {
-        const Cluster &k = e->cl[c];
-        rec.resize((size_t)k.n * e->R);
-        ce = cudaMemcpy(rec.data(), e->d_jp + (size_t)k.off * e->R, rec.size() * sizeof(double),
-                        cudaMemcpyDeviceToHost);
-        if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "init read", ce);
-        for (int i = 0; i < k.n; ++i) {
-            double *r = rec.data() + (size_t)i * e->R;
-            r[7] = tsys;
-            std::memset(r + 8, 0, sizeof(double) * (e->R - 8));
-        }
-        ce = cudaMemcpy(e->d_jp + (size_t)k.off * e->R, rec.data(), rec.size() * sizeof(double),
-                        cudaMemcpyHostToDevice);
-        if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "init write", ce);
-    }
     ce = cudaMemcpy(e->d_cl, e->cl.data(), e->cl.size() * sizeof(Cluster), cudaMemcpyHostToDevice);
     if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "cluster table", ce);
+    // tlast = tsys, derivatives zero, for every real slot
+    ens_reset_kernel<<<e->nslot / kClusterPad, kClusterPad, 0, e->stream>>>(e->d_jp, e->R, e->d_cl,
+                                                                          e->d_slot_cluster, tsys);
+    ce = cudaGetLastError();
+    if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "record reset", ce);
     EnsSched &s = *e->h_s;
     std::memset(&s, 0, sizeof(EnsSched));
     s.tnext_bits = kInf;
@@ -1138,20 +1165,6 @@ int hb_ens_init(hb_ens *e, double tsys, double eta, double eta_s, double dtmax)
     ce = cudaMemcpy(e->d_cstate, cs.data(), cs.size() * sizeof(TeamState), cudaMemcpyHostToDevice);
     if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "cluster state", ce);
     e->groups_ready = false;
-    ce = cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal);
-    if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "capture", ce);
-    cudaError_t le = cudaSuccess;
-    for (int k = 0; k < kEnsStepsPerGraph && le == cudaSuccess; ++k) le = dispatch_step(e);
-    cudaGraph_t g = nullptr;
-    ce = cudaStreamEndCapture(e->stream, &g);
-    if (le != cudaSuccess || ce != cudaSuccess) {
-        if (g) cudaGraphDestroy(g);
-        return ens_fail(e, HB_ERR_CUDA, "capturing the ensemble step graph",
-                        le != cudaSuccess ? le : ce);
-    }
-    e->graph = g;
-    ce = cudaGraphInstantiate(&e->exec, g, 0);
-    if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "instantiate", ce);
     e->ready = true;
     return HB_OK;
 }
@@ -1174,6 +1187,8 @@ int hb_ens_run(hb_ens *e, double tend, long long max_block_steps)
 
     // the lockstep engine: the other clusters (those already at tend have
     // no active particles until tend)
+    s0 = ensure_graph(e);
+    if (s0 != HB_OK) return s0;
     volatile EnsStatus *st = e->h_st;
     if (!(tend >= st->tsys)) return ens_fail(e, HB_ERR_INVALID, "tend is before tsys");
     ce = cudaMemcpy(&e->d_s->tend, &tend, sizeof(double), cudaMemcpyHostToDevice);
