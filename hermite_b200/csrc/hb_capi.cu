@@ -872,7 +872,7 @@ int setup_integrator(hb_ctx *ctx, double tsys, double eps2, double eta, double d
     HB_CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t ce = cudaSuccess;
     for (int k = 0; k < kStepsPerGraph && ce == cudaSuccess; ++k)
-        ce = integrator_step_launch(ctx->order, L, k & 1, ctx->stream);
+        ce = integrator_step_launch(ctx->order, L, k & 1, k == kStepsPerGraph - 1, ctx->stream);
     cudaGraph_t graph = nullptr;
     const cudaError_t ee = cudaStreamEndCapture(ctx->stream, &graph);
     if (ce != cudaSuccess || ee != cudaSuccess) {

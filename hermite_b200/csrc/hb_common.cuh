@@ -129,10 +129,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
 // now, then wait until the previous kernel's results are visible.  (Between
 // kernels launched with programmatic stream serialisation; otherwise both
 // instructions are no-ops.)
+__device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter()
 {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_launch_next();
+    pdl_wait();
 }
 
 __device__ __forceinline__ void raise_error(int *err, int code)

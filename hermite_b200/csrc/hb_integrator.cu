@@ -53,9 +53,10 @@ struct StepArgs {
 // shape has 4 to 16 chunks, one to four per warp in turn (0.7 us each); with
 // more slices the sum in the corrector grows.  The bounds are flat: halving or
 // doubling any of them moves the mean step by at most 3 % (N = 2500 ... 131072,
-// 4th to 8th order).
+// 4th to 8th order); slices of one chunk, a quarter of it per warp, measured 1 us
+// slower at N = 512 ... 8192 (the sum grows by more than the chain shrinks).
 //
-// Per block step, 4th order, N = 4096 / 16384 / 65536: 12.8 / 27.6 / 116 us, from
+// Per block step, 4th order, N = 4096 / 16384 / 65536: 12.6 / 25.6 / 112 us, from
 // 18.4 / 34.0 / 125 us with five kernels, raw records predicted by every item and
 // the last CTA of an i-tile adding its slices.
 struct StepSplit {
@@ -73,8 +74,8 @@ __device__ __forceinline__ StepSplit step_split(int nact, const StepArgs &a)
     int c = r.wj == 4 ? 4 * max(1, min(4, (int)fmaxf(sqrtf(x), a.nchunk / 1024.0f))) : 8;
     c = max(c, (int)(x * 0.125f));
     r.S = max(1, a.nchunk / c);
-    const long long smax = (long long)(a.partial_cap / ((size_t)r.gx * r.ti * F));
-    r.S = (int)max(1ll, min((long long)r.S, smax));
+    const size_t row = (size_t)r.gx * r.ti * F;
+    if (r.S * row > a.partial_cap) r.S = (int)max((size_t)1, a.partial_cap / row);
     return r;
 }
 
@@ -199,6 +200,7 @@ __device__ __forceinline__ bool force_phase(const StepArgs &a, int par, unsigned
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ig = warp / sp.wj, jg = warp % sp.wj;
     const int items = sp.gx * sp.S;
+    const int len = a.nchunk / sp.S, rem = a.nchunk % sp.S;     // chunks of a slice, one more in the first rem
     const size_t ispan = (size_t)sp.gx * sp.ti;
     double *out = sp.S == 1 ? a.force : a.partial;
     // FP64 steps of at most kLanesMaxAct active slots: lanes share an
@@ -208,8 +210,7 @@ __device__ __forceinline__ bool force_phase(const StepArgs &a, int par, unsigned
 
     for (int item = blockIdx.x; item < items;) {
         const int itile = item / sp.S, sl = item % sp.S;
-        const int c0 = (int)(((long long)sl * a.nchunk) / sp.S);
-        const int c1 = (int)(((long long)(sl + 1) * a.nchunk) / sp.S);
+        const int c0 = sl * len + min(sl, rem), c1 = c0 + len + (sl < rem ? 1 : 0);
         const int ntile = (c1 - c0 + TCH - 1) / TCH;
         auto issue = [&](int t) {   // thread 0 only
             const unsigned gt = g + t;
@@ -300,7 +301,7 @@ __device__ __forceinline__ bool force_phase(const StepArgs &a, int par, unsigned
 template <int ORDER, bool MIXED>
 __global__ void __launch_bounds__(kStepThreads, 4) step_force_kernel(StepArgs a, int par)
 {
-    pdl_enter();
+    pdl_wait();
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + StepShape<ORDER, MIXED>::body_bytes);
     if (threadIdx.x == 0) {
@@ -311,6 +312,20 @@ __global__ void __launch_bounds__(kStepThreads, 4) step_force_kernel(StepArgs a,
     __syncthreads();
     unsigned g = 0;   // tiles issued by this CTA so far (mbarrier phases)
     force_phase<ORDER, MIXED>(a, par, smem, bar, g);
+    // not before the items are taken: the corrector's waiting CTAs would hold
+    // registers that this kernel's need (2-3 % of the mean step at N = 65536)
+    pdl_launch_next();
+}
+
+// What the host reads between replays.  A step's end would wait for the writes
+// to cross the host link, so only the last step of a replay reports.
+__device__ __forceinline__ void report_status(const Sched *s)
+{
+    IntStatus *st = s->status;
+    st->tsys = s->tsys;
+    st->particle_steps = s->particle_steps;
+    st->block_steps = s->block_steps;
+    st->error = s->error;
 }
 
 // Phase 3: slices summed, corrector, and the next block time.  L lanes (a
@@ -319,7 +334,7 @@ __global__ void __launch_bounds__(kStepThreads, 4) step_force_kernel(StepArgs a,
 // alone, not on the particle's place in the active list, which the compaction
 // does not fix.
 template <int ORDER>
-__device__ __forceinline__ void correct_phase(const StepArgs &a, int par)
+__device__ __forceinline__ void correct_phase(const StepArgs &a, int par, bool report)
 {
     constexpr int R = Rec<ORDER>::words, F = Frc<ORDER>::words;
     Sched *s = a.s;
@@ -400,19 +415,15 @@ __device__ __forceinline__ void correct_phase(const StepArgs &a, int par)
             s->particle_steps += nact;
             s->block_steps += 1;
         }
-        IntStatus *st = s->status;
-        st->tsys = s->tsys;
-        st->particle_steps = s->particle_steps;
-        st->block_steps = s->block_steps;
-        st->error = s->error;
+        if (report) report_status(s);
     }
 }
 
 template <int ORDER>
-__global__ void __launch_bounds__(kCorrectThreads) step_correct_kernel(StepArgs a, int par)
+__global__ void __launch_bounds__(kCorrectThreads) step_correct_kernel(StepArgs a, int par, int report)
 {
     pdl_enter();
-    correct_phase<ORDER>(a, par);
+    correct_phase<ORDER>(a, par, report != 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -510,17 +521,14 @@ persistent_kernel(PersistArgs p)
         const int par = (int)(k & 1);
         const bool live = active_phase<ORDER, MIXED>(a, par);
         if (!grid_barrier(p.gbar, p.spin)) { gave_up = true; break; }
-        if (!live) {                     // every CTA reads the same state
-            if (blockIdx.x == 0 && threadIdx.x == 0)
-                s->status->error = s->error;   // an error set after the last status write
-            return;
-        }
+        if (!live) break;                // every CTA reads the same state
         if (!force_phase<ORDER, MIXED>(a, par, smem, bar, g))
             return;                      // raised; the others give up at the next barrier
         if (!grid_barrier(p.gbar, p.spin)) { gave_up = true; break; }
-        correct_phase<ORDER>(a, par);
+        correct_phase<ORDER>(a, par, false);
         if (!grid_barrier(p.gbar, p.spin)) { gave_up = true; break; }
     }
+    if (!gave_up && blockIdx.x == 0 && threadIdx.x == 0) report_status(s);
     if (gave_up && threadIdx.x == 0) {   // a barrier wait gave up
         s->error = 2;
         raise_error(a.err, kErrWaitTimeout);
@@ -597,7 +605,7 @@ static StepArgs step_args(const IntegratorLaunch &L)
 // One (order, precision) instance of the step's kernels.
 template <int ORDER, bool MIXED>
 struct StepKernels {
-    static cudaError_t launch(const IntegratorLaunch &L, int par, cudaStream_t s)
+    static cudaError_t launch(const IntegratorLaunch &L, int par, bool report, cudaStream_t s)
     {
         const StepArgs a = step_args(L);
         const int nb = std::min(L.nchunk / 4, L.nsm * 16);       // 128 slots per CTA
@@ -607,7 +615,7 @@ struct StepKernels {
                            StepShape<ORDER, MIXED>::smem_bytes, s, a, par);
         if (e == cudaSuccess)
             e = launch_pdl(step_correct_kernel<ORDER>, dim3(std::max(1, std::min(L.nchunk / 4, L.nsm * 2))),
-                           kCorrectThreads, 0, s, a, par);
+                           kCorrectThreads, 0, s, a, par, report ? 1 : 0);
         return e;
     }
     static cudaError_t start(const IntegratorLaunch &L, cudaStream_t s)
@@ -656,9 +664,9 @@ static cudaError_t with_step(int order, bool mixed, Fn fn)
     return cudaErrorInvalidValue;
 }
 
-cudaError_t integrator_step_launch(int order, const IntegratorLaunch &L, int par, cudaStream_t s)
+cudaError_t integrator_step_launch(int order, const IntegratorLaunch &L, int par, bool report, cudaStream_t s)
 {
-    return with_step(order, L.mixed, [&](auto k) { return decltype(k)::launch(L, par, s); });
+    return with_step(order, L.mixed, [&](auto k) { return decltype(k)::launch(L, par, report, s); });
 }
 
 cudaError_t integrator_start(int order, const IntegratorLaunch &L, cudaStream_t s)

@@ -60,8 +60,8 @@ struct ForceVariant {
 };
 
 // Device-resident block-step integration (hb_integrator.cu).
-// What the host reads between graph replays; written once per block step by
-// one thread into mapped pinned memory (the scheduler itself stays in device
+// What the host reads between graph replays; written by the last block step of
+// each by one thread into mapped pinned memory (the scheduler itself stays in device
 // memory: its atomics must not cross the host link).
 struct IntStatus {
     double tsys;
@@ -104,8 +104,9 @@ struct IntegratorLaunch {
 // Before a run: tlast + dt per slot, the first block time, counters.
 cudaError_t integrator_start(int order, const IntegratorLaunch &L, cudaStream_t s);
 // One block step; par alternates between 0 and 1, starting with 0 after
-// integrator_start.
-cudaError_t integrator_step_launch(int order, const IntegratorLaunch &L, int par, cudaStream_t s);
+// integrator_start; report: write the status the host reads.
+cudaError_t integrator_step_launch(int order, const IntegratorLaunch &L, int par, bool report,
+                                   cudaStream_t s);
 
 // Persistent engine (hb_integrator.cu): one cooperative launch runs up to
 // max_steps block steps (an even number, except the last launch before an
