@@ -240,11 +240,18 @@ const TuneEntry *lookup_tuning(int order, bool mixed, int n, int nact)
 // takes in turn; it wins up to 64 particles and where all pairs together are
 // few (N = 32768, 6th order, nact = 300: 48.6 against 51.3 us; N = 262144,
 // nact = 500: 493 against 480 us).
-constexpr int kShapeWide = 8, kShapeNarrow = 11;
+//
+// Up to 3072 slots the launches themselves matter: shape 13 (four warps, 32
+// particles) predicts what it streams and saves the predictor's launch (block
+// steps of N = 600, 8th order, nact = 17: 31.7 against 36.9 us; N = 1346, nact = 336 35.6
+// against 40.0; N = 4000, all active 229 against 221).
+constexpr int kShapeWide = 8, kShapeNarrow = 11, kShapeFused = 13;
 constexpr long long kNarrowUnits = 12288;      // 64-particle tiles x chunks
+constexpr int kFusedSlots = 3072;
 
 int auto_variant(const hb_ctx *c, int nact)
 {
+    if (c->npad <= kFusedSlots) return kShapeFused;
     const long long units = (long long)((nact + 63) / 64) * (c->npad / 32);
     return nact <= 64 || units <= kNarrowUnits ? kShapeNarrow : kShapeWide;
 }
@@ -253,12 +260,19 @@ int auto_variant(const hb_ctx *c, int nact)
 int auto_slices(int v, int gx, int nchunk, int resident)
 {
     const double x = (double)gx * nchunk / resident;       // chunks per resident CTA
-    // Large steps: 8 waves, slices of at least 8 chunks.  Small ones (the
-    // narrow shape): a CTA takes about 0.7 us per chunk in turn, and the reduce
-    // grows with the slices, past 256 of them most; the rule is within 2 us of
-    // the best of c = 1, 2, 4, 8 over 4th to 8th order, N = 1024 ... 262144.
-    double c = 8.0;
-    if (v == kShapeNarrow) c = std::max(1.0, std::min(8.0, std::max(2.0 * std::sqrt(x), nchunk / 256.0)));
+    // Large steps: 8 waves, slices of at least 8 chunks (4 where that leaves
+    // less than two waves, but at most 1024 slices).  Small ones, in the narrow
+    // shape: an even number of chunks for its two warps, 0.7 us each, against a
+    // reduce that grows with the slices, past 256 of them most.  The rule is within
+    // 3 us or 3 % of the best of c = 1, 2, 4, 8 over 4th to 8th order, N = 600 ... 262144
+    // (8th order, N = 2500, nact = 625: 49.4 us; slices of 3 and 4 chunks in turn 61.3).
+    double c;
+    if (v == kShapeFused)
+        c = 4;           // one per warp
+    else if (v == kShapeNarrow)
+        c = 2 * std::max(1, std::min(4, std::max((int)(0.6 * std::sqrt(x) + 0.5), nchunk / 512)));
+    else
+        c = x < 16.0 ? std::max(4, std::min(8, nchunk / 1024)) : 8;
     c = std::max(c, x / 8.0);
     return std::max(1, (int)(nchunk / c));
 }

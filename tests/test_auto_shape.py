@@ -1,7 +1,8 @@
 """The automatic launch shape (two-warp CTAs, many j-slices, a separate sum of
 the slices) against the oracle at the sizes where its tiling changes: one i
-past a tile, one chunk, slices that do not divide the chunks, both shapes
-(narrow up to 64 active particles and for small problems, wide past them).
+past a tile, one chunk, slices that do not divide the chunks, and each shape
+(fused up to 3072 slots, narrow up to 64 active particles and for small
+problems, wide past them).
 Tolerances as tests/test_gpu_parity.py: summation order only in FP64.
 """
 import numpy as np
@@ -21,6 +22,8 @@ TOL = {"fp64": [1e-12] * 4, "mixed": [1e-6, 1e-5, 1e-4, 1e-2]}
 @pytest.mark.parametrize("n,nacts", [
     (17, [17]),                       # one chunk group, one slice
     (300, [17, 33, 64, 65, 300]),     # fewer chunks than slices are wanted
+    (3072, [17, 100, 3072]),          # the last size that predicts as it streams
+    (3073, [17, 65, 3073]),           # the first with a predictor pass
     (8200, [17, 65, 129, 600]),       # the padded tail in the last slice
     (70000, [31, 64, 65, 700]),       # the wide shape past 64
 ])
