@@ -25,15 +25,19 @@ cudaError_t launch_t(const ForceArgs &f, size_t cap, int nsm, cudaStream_t s, in
     const int groups = (a.ca + GC - 1) / GC;
     const long long chunk = F * 32, room = (long long)(cap / chunk);   // scratch in [F][32] blocks
     for (int g0 = 0; g0 < groups; g0 += a.ng) {
-        // about 6 waves of CTAs: a CTA's chunks, in whole tiles (3 and 12 waves
-        // measured 2-5 % slower)
-        const long long wide = std::max(1LL, std::min((long long)groups - g0, room / a.ca));
-        const long long units = wide * (a.nchunk - (long long)g0 * GC);
-        const long long lc = units / (6LL * SymShape<ORDER>::MINB * nsm);
+        // as many groups as the scratch has rows and slice sums for, in slices
+        // that make about 10 waves of CTAs, in whole tiles (6th order, N = 131072:
+        // 4 waves 41.7 ms, 6 40.5, 10 40.0, 16 40.0; N = 50000 6.37, 6.09, 6.12, 6.34)
         a.g0 = g0;
-        a.lc = (int)std::max(1LL, (lc + kSymFTile - 1) / kSymFTile) * kSymFTile;
-        a.smax = sym_slices(a.nchunk, g0, GC, a.lc);
-        a.ng = (int)std::min((long long)(groups - g0), room / (a.ca + (long long)a.smax * GC));
+        a.ng = (int)std::min((long long)(groups - g0), room / a.ca);
+        for (int pass = 0; pass < 3; ++pass) {
+            if (a.ng < 1) return cudaErrorInvalidValue;
+            const long long units = (long long)a.ng * (a.nchunk - (long long)g0 * GC) - (long long)GC * a.ng * (a.ng - 1) / 2;
+            const long long lc = units / (10LL * SymShape<ORDER>::MINB * nsm);
+            a.lc = (int)std::max(1LL, (lc + kSymFTile - 1) / kSymFTile) * kSymFTile;
+            a.smax = sym_slices(a.nchunk, g0, GC, a.lc);
+            a.ng = (int)std::min((long long)a.ng, room / (a.ca + (long long)a.smax * GC));
+        }
         if (a.ng < 1) return cudaErrorInvalidValue;
         a.rows = f.partial;
         a.cols = f.partial + (size_t)a.ng * a.ca * chunk;
@@ -53,7 +57,7 @@ cudaError_t launch_t(const ForceArgs &f, size_t cap, int nsm, cudaStream_t s, in
 
 // Both sides measured (ms, ordered pairs / pairs once): all of N = 4096 0.060 /
 // 0.049 at 4th order and 0.088 / 0.090 at 6th, 12000 0.526 / 0.425 (6th), 131072
-// 59.9 / 41.4 (6th); parts of N = 131072 at 6th order: 20000 8.93 / 8.94,
+// 59.9 / 40.0 (6th); parts of N = 131072 at 6th order: 20000 8.93 / 8.94,
 // 45000 20.0 / 19.2, 70000 31.3 / 27.5; of 65536 at 4th: 20000 2.61 / 2.69, 30000
 // 3.90 / 3.69.  The 8th-order sums are compensated; they keep ordered pairs.
 bool force_sym_takes(int order, bool mixed, int nact, int npad, size_t cap)

@@ -22,12 +22,12 @@
 // j-slices; sym_band_kernel adds a band's rows and slices to the forces in a fixed
 // order, so results are deterministic.
 //
-// What bounds it: the FP64 pipe (70 % busy over the whole call) beside the
+// What bounds it: the FP64 pipe (76 % busy while an SM has CTAs) beside the
 // j-states' loads and the shuffles, 20 + 18 shared-memory cycles per step at 6th
 // order for 3 x 63 FP64 instructions: with one i-chunk per warp those bound it (339
-// Gint/s at N = 131072), with two 401, three 415, four 418, five 389 (spills);
-// ordered pairs 292.  4th order, N = 65536: 675 against 505.  A band's sums are
-// 2-3 % of the time.
+// Gint/s at N = 131072), with two 401, three 415, four 418, five 389 (spills), all
+// with 6 waves; 429 with 10.  Ordered pairs 292.  4th order, N = 65536: 715 against
+// 505.  A band's sums and its last CTAs are about 5 % of the time.
 #pragma once
 #include "hb_common.cuh"
 #include "hb_force.cuh"
