@@ -527,9 +527,12 @@ int hb_create(int order, int nbody, int precision, hb_ctx **out)
     const size_t pred_bytes = std::max(np * pred64_ncomp(order) * sizeof(double),
                                        np * predmx_ncomp(order) * sizeof(float));
     // j-slices' partials; or rows of one double per value and slot for pairs
-    // taken once, 32 rows up to 256 MiB (16 rows: 4-6 % slower at N = 50000 ... 65536)
-    ctx->partial_cap = std::max((size_t)2 * ctx->nsm * 8 * 256 * ctx->F,
-                                std::min(32 * np * ctx->F, (size_t)32 << 20));
+    // taken once: 64 rows up to 512 MiB (32 rows up to 256 MiB: 3-7 % slower at N =
+    // 20000 ... 65536, 1 % at 131072), and 64 MiB from 4096 slots on, which
+    // takes 8192 in one launch (0.124 ms at 4th order; in two, 0.153)
+    const size_t slices_cap = (size_t)2 * ctx->nsm * 8 * 256 * ctx->F;
+    ctx->partial_cap = std::max(slices_cap, std::min(64 * np * ctx->F, (size_t)64 << 20));
+    if (np >= 4096) ctx->partial_cap = std::max(ctx->partial_cap, (size_t)8 << 20);
     bool ok = true;
     ok = ok && cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&ctx->ev_upload, cudaEventDisableTiming) == cudaSuccess;
@@ -542,9 +545,14 @@ int hb_create(int order, int nbody, int precision, hb_ctx **out)
     ok = ok && cudaMalloc((void **)&ctx->d_force, np * ctx->F * sizeof(double)) == cudaSuccess;
     ok = ok && cudaMalloc((void **)&ctx->d_pot, np * sizeof(double)) == cudaSuccess;
     ok = ok && cudaMalloc((void **)&ctx->d_posm, np * (order == 9 ? 7 : 4) * sizeof(double)) == cudaSuccess;
-    ok = ok && cudaMalloc((void **)&ctx->d_partial, ctx->partial_cap * sizeof(double)) == cudaSuccess;
     ok = ok && cudaMalloc(&ctx->d_pred, pred_bytes) == cudaSuccess;
     ok = ok && cudaMalloc((void **)&ctx->d_counter, (np / 32 + 1) * sizeof(unsigned)) == cudaSuccess;
+    if (ok && cudaMalloc((void **)&ctx->d_partial, ctx->partial_cap * sizeof(double)) != cudaSuccess) {
+        // little memory left: room for the slices only (fewer rows, or ordered pairs)
+        (void)cudaGetLastError();
+        ctx->partial_cap = slices_cap;
+        ok = cudaMalloc((void **)&ctx->d_partial, ctx->partial_cap * sizeof(double)) == cudaSuccess;
+    }
     if (ok) {
         ok = cudaHostGetDevicePointer((void **)&ctx->d_err, ctx->h_err, 0) == cudaSuccess &&
              cudaHostGetDevicePointer((void **)&ctx->h_force_dev, ctx->h_force, 0) == cudaSuccess;

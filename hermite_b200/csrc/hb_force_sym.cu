@@ -26,14 +26,18 @@ cudaError_t launch_t(const ForceArgs &f, size_t cap, int nsm, cudaStream_t s, in
     const long long chunk = F * 32, room = (long long)(cap / chunk);   // scratch in [F][32] blocks
     for (int g0 = 0; g0 < groups; g0 += a.ng) {
         // as many groups as the scratch has rows and slice sums for, in slices
-        // that make about 10 waves of CTAs, in whole tiles (6th order, N = 131072:
-        // 4 waves 41.7 ms, 6 40.5, 10 40.0, 16 40.0; N = 50000 6.37, 6.09, 6.12, 6.34)
+        // that make 10 to 20 waves of CTAs, in whole tiles: 20 as long as the slice
+        // sums take no more than 0.4 of the rows' room (with 32 rows, 6th order, N =
+        // 131072: 4 waves 41.7 ms, 6 40.5, 10 40.0; with 64, 10 39.7, 20 39.3; N =
+        // 50000 5.92, 5.98)
         a.g0 = g0;
         a.ng = (int)std::min((long long)(groups - g0), room / a.ca);
         for (int pass = 0; pass < 3; ++pass) {
             if (a.ng < 1) return cudaErrorInvalidValue;
             const long long units = (long long)a.ng * (a.nchunk - (long long)g0 * GC) - (long long)GC * a.ng * (a.ng - 1) / 2;
-            const long long lc = units / (10LL * SymShape<ORDER>::MINB * nsm);
+            const long long wave = SymShape<ORDER>::MINB * nsm;
+            const long long lc = std::min(units / (10 * wave),
+                                          std::max(units / (20 * wave), 5LL * GC * a.nchunk / (2 * a.ca)));
             a.lc = (int)std::max(1LL, (lc + kSymFTile - 1) / kSymFTile) * kSymFTile;
             a.smax = sym_slices(a.nchunk, g0, GC, a.lc);
             a.ng = (int)std::min((long long)a.ng, room / (a.ca + (long long)a.smax * GC));
@@ -55,16 +59,19 @@ cudaError_t launch_t(const ForceArgs &f, size_t cap, int nsm, cudaStream_t s, in
 
 }  // namespace
 
-// Both sides measured (ms, ordered pairs / pairs once): all of N = 4096 0.060 /
-// 0.049 at 4th order and 0.088 / 0.090 at 6th, 12000 0.526 / 0.425 (6th), 131072
-// 59.9 / 40.0 (6th); parts of N = 131072 at 6th order: 20000 8.93 / 8.94,
-// 45000 20.0 / 19.2, 70000 31.3 / 27.5; of 65536 at 4th: 20000 2.61 / 2.69, 30000
-// 3.90 / 3.69.  The 8th-order sums are compensated; they keep ordered pairs.
+// The share of the pairs that is one-sided grows as fewer particles are active, and
+// small calls do not fill the waves.  Both sides measured (ms, ordered pairs /
+// pairs once): all of N = 4096 0.060 / 0.049 at 4th order and 0.088 / 0.090 at
+// 6th, 131072 59.9 / 39.0 (6th); a fifth of N = 40000 0.656 / 0.640 (4th) and
+// 1.122 / 1.090 (6th), of 262144 47.1 / 44.0 (6th), 0.15 of 65536 1.291 / 1.302
+// (4th); 4096 of 16384 0.155 / 0.157 (4th) and 0.252 / 0.259 (6th).  The 8th-order
+// sums are compensated; they keep ordered pairs.
 bool force_sym_takes(int order, bool mixed, int nact, int npad, size_t cap)
 {
     if (mixed || (order != 4 && order != 6)) return false;
     const size_t blocks = cap / (size_t)(3 * (order / 2) * 32);
-    return nact >= 4096 && nact >= npad * 4LL / 10 && blocks >= (size_t)npad / 32 * 2;
+    const bool most = nact >= 4096 && nact >= npad * 4LL / 10, many = nact >= 8192 && nact >= npad / 5;
+    return (most || many) && blocks >= (size_t)npad / 32 * 2;
 }
 
 cudaError_t launch_force_sym(int order, const ForceArgs &f, size_t cap, int nsm, cudaStream_t s, int *launches)

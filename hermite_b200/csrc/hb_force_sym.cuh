@@ -26,8 +26,8 @@
 // j-states' loads and the shuffles, 20 + 18 shared-memory cycles per step at 6th
 // order for 3 x 63 FP64 instructions: with one i-chunk per warp those bound it (339
 // Gint/s at N = 131072), with two 401, three 415, four 418, five 389 (spills), all
-// with 6 waves; 429 with 10.  Ordered pairs 292.  4th order, N = 65536: 715 against
-// 505.  A band's sums and its last CTAs are about 5 % of the time.
+// with 6 waves and 16 rows; 440 with 20 and 64.  Ordered pairs 292.  4th order, N =
+// 65536: 741 against 505.  A band's sums and its last CTAs are 2-3 % of the time.
 #pragma once
 #include "hb_common.cuh"
 #include "hb_force.cuh"
@@ -102,6 +102,7 @@ template <int ORDER>
 struct SymShape {
     static constexpr int NI = ORDER == 4 ? 4 : 3;   // i-chunks per warp
     static constexpr int MINB = 2;                 // CTAs per SM
+    static constexpr int unroll = ORDER == 4 ? 2 : 8;   // steps; all of 1, 2, 4, 8 within 2 %
     static constexpr int GC = kSymFWarps * NI;            // chunks of a group
     static constexpr int F = Frc<ORDER>::words, CB = Pred64<ORDER>::chunk_bytes;
     static constexpr int tile_bytes = kSymFTile * CB;
@@ -117,6 +118,7 @@ force_sym_kernel(const SymArgs a)
     pdl_enter();
     using Sh = SymShape<ORDER>;
     constexpr int F = Sh::F, NC = Pred64<ORDER>::ncomp, NI = Sh::NI, GC = Sh::GC, T = kSymFWarps * 32;
+    constexpr int UNROLL = Sh::unroll;
     extern __shared__ __align__(128) unsigned char smem[];
     double *accj = reinterpret_cast<double *>(smem + Sh::acc_off);
     uint64_t *bar = reinterpret_cast<uint64_t *>(smem + Sh::bar_off);
@@ -180,7 +182,7 @@ force_sym_kernel(const SymArgs a)
             for (int c = 0; c < F; ++c) fj[c] = 0.0;
             const int next = (lane + 1) & 31;
             int jl = lane;
-#pragma unroll 4
+#pragma unroll UNROLL
             for (int st = 0; st < 32; ++st) {
                 Body64 J;
                 load_i64<ORDER>(cp, 0, jl, J);
