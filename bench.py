@@ -54,6 +54,9 @@ ORDER, N, EPS = 6, 262144, 1.0 / 4096
 CPU_NACT = 8192            # i-particles of the CPU sample of the step
 NSAMPLE = 4096             # i-particles of the accuracy sample
 FLOPS = {4: 60, 6: 97, 8: 144}
+# the FP64 kernel takes each pair of active particles once (6th order): the
+# pair's 97 flops serve one particle, m_i/r^3 and nine FMAs more the other
+PAIR_FLOPS = FLOPS[ORDER] + 19
 L2_FLUSH_BYTES = 256 << 20
 
 
@@ -262,10 +265,10 @@ def traffic_from_profiles(name):
 
 
 def tiled_shape(order, n, nact):
-    """The tiled force kernel's shape (variant, j-slices) that the library
-    takes from its tuning table for (order, FP64, n, nact): the nearest N
-    bucket, then the nearest nact bucket, the slice count rescaled to the
-    bucket's CTA count (hb_capi.cu, pick_variant)."""
+    """The tiled force kernel's shape (variant, j-slices) in the library's
+    tuning table for (order, FP64, n, nact): the nearest N bucket, then the
+    nearest nact bucket, the slice count rescaled to the bucket's CTA count
+    (hb_capi.cu, pick_variant)."""
     import ctypes
     import math
     from hermite_b200 import load_library
@@ -399,11 +402,12 @@ def run_ours(args):
     fp64_peak = measure_fma_peak(0)      # GFLOP/s, same device, same run
     fp32_peak = measure_fma_peak(2)
     force_avg_ms = sum(force_ms) / len(force_ms)
-    achieved = nint * FLOPS[ORDER] / (force_avg_ms * 1e-3) * 1e-12
+    npair = N * (N + 1) // 2
+    achieved = npair * PAIR_FLOPS / (force_avg_ms * 1e-3) * 1e-12
     mforce_avg_ms = sum(mforce_ms) / len(mforce_ms)
     machieved = nint * FLOPS[ORDER] / (mforce_avg_ms * 1e-3) * 1e-12
     mvalue = nint * args.steps / (sum(mstep_ms) * 1e-3) * 1e-9
-    traffic = traffic_from_profiles("force_fp64_o6_n262144.txt")
+    traffic = traffic_from_profiles("force_sym_o6_n262144.txt")
     mtraffic = traffic_from_profiles("force_mixed_o6_n262144.txt")
 
     # the accuracy, 8th-order, integrator, ensemble and CPU legs run on
@@ -464,11 +468,11 @@ def run_ours(args):
         "gpu_launches": launches,
         "roofline": {"bound": "fp64", "achieved": achieved, "peak": fp64_peak * 1e-3,
                      "unit": "TFLOP/s", "frac": achieved / (fp64_peak * 1e-3), "traffic": traffic,
-                     "kernel": "hb::force_kernel<6, FP64>",
+                     "kernel": "hb::force_sym_kernel<6>",
                      "peak_source": "FP64 FMA-chain kernel measured in this run "
                                     "(hb_measure_fma_peak); MEASURED_PEAKS.json has no FP64 figure",
-                     "achieved_basis": f"N^2 x {FLOPS[ORDER]} flops per launch / mean CUDA-event "
-                                       "duration of the force launch"},
+                     "achieved_basis": f"N(N+1)/2 pairs x {PAIR_FLOPS} flops, each pair taken once for "
+                                       "both particles / mean CUDA-event duration of the force"},
         "kernel_ms": {"predict": sum(pred_ms) / len(pred_ms), "force": force_avg_ms},
         "fp32_peak_tflops": fp32_peak * 1e-3,
         "mixed": mixed,
