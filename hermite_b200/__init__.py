@@ -46,7 +46,7 @@ EXPORTED_SYMBOLS = (
     "hb_predict_all_device", "hb_predict_pass", "hb_force_device", "hb_download_forces", "hb_device_forces",
     "hb_synchronize", "hb_launch_count", "hb_set_force_shape", "hb_set_wait_limit",
     "hb_force_variant_count",
-    "hb_force_variant_info", "hb_measure_fma_peak", "hb_force_predicted_noalloc",
+    "hb_force_variant_info", "hb_force_pairs_once_bands", "hb_measure_fma_peak", "hb_force_predicted_noalloc",
     "hb_integrator_init", "hb_integrator_run", "hb_integrator_stats", "hb_energy",
     "hb_integrator_set_engine", "hb_integrator_engine",
     "hb_get_records", "hb_ens_create", "hb_ens_destroy", "hb_ens_last_error",
@@ -163,6 +163,7 @@ def load_library() -> ctypes.CDLL:
         "hb_force_variant_count": (I, [I, I]),
         "hb_force_variant_info": (I, [I, I, I, ctypes.POINTER(I), ctypes.POINTER(I),
                                       ctypes.POINTER(I)]),
+        "hb_force_pairs_once_bands": (I, [I, I, I, ctypes.c_longlong]),
         "hb_measure_fma_peak": (I, [I, dp]),
         "hb_force_predicted_noalloc": (I, [I, I, P, I, I, D, P, P]),
         "hb_integrator_init": (I, [P, D, D, D, D, D]),

@@ -810,6 +810,12 @@ int hb_force_variant_info(int order, int precision, int variant, int *threads, i
     return HB_OK;
 }
 
+int hb_force_pairs_once_bands(int order, int n, int nact, long long doubles)
+{
+    if (!valid_order(order) || n < 1 || nact < 0 || nact > n || doubles < 0) return HB_ERR_INVALID;
+    return force_sym_bands(order, nact, (n + kSlotPad - 1) / kSlotPad * kSlotPad, (size_t)doubles, 148);
+}
+
 // ---- device-resident integration -------------------------------------------
 namespace {
 constexpr int kStepsPerGraph = 32;      // even: the steps' two counters take turns

@@ -6,6 +6,48 @@
 namespace hb {
 namespace {
 
+struct Band {
+    int ng, lc, smax;      // groups, chunks per slice, slices per group at most
+};
+
+// The band from group g0 on, for scratch of `room` [F][32] blocks: as many groups as
+// it has rows and slice sums for, in slices that make 10 to 20 waves of CTAs, in
+// whole tiles: 20 as long as the slice sums take no more than 0.4 of the rows' room
+// (with 32 rows, 6th order, N = 131072: 4 waves 41.7 ms, 6 40.5, 10 40.0; with 64,
+// 10 39.7, 20 39.3; N = 50000 5.92, 5.98).  Little scratch makes the slices longer:
+// a group's row and its slice sums fit wherever two rows do.
+template <int ORDER>
+Band band_from(int g0, int ca, int nchunk, long long room, int nsm)
+{
+    constexpr int GC = SymShape<ORDER>::GC;
+    const int groups = (ca + GC - 1) / GC;
+    const long long wave = SymShape<ORDER>::MINB * nsm, most = (room - ca) / GC;
+    Band b{(int)std::min((long long)(groups - g0), room / ca), 0, 0};
+    if (most < 1) return Band{};
+    for (int pass = 0; pass < 3 && b.ng > 0; ++pass) {
+        const long long units = (long long)b.ng * (nchunk - (long long)g0 * GC) - (long long)GC * b.ng * (b.ng - 1) / 2;
+        long long lc = std::min(units / (10 * wave), std::max(units / (20 * wave), 5LL * GC * nchunk / (2 * ca)));
+        lc = std::max({lc, (nchunk - (long long)g0 * GC + most - 1) / most, 1LL});
+        b.lc = (int)((lc + kSymFTile - 1) / kSymFTile) * kSymFTile;
+        b.smax = sym_slices(nchunk, g0, GC, b.lc);
+        b.ng = (int)std::min((long long)b.ng, room / (ca + (long long)b.smax * GC));
+    }
+    return b;
+}
+
+template <int ORDER>
+int bands_t(int ca, int nchunk, size_t cap, int nsm)
+{
+    const long long room = (long long)(cap / (Frc<ORDER>::words * 32));
+    int bands = 0;
+    for (int g0 = 0; g0 * SymShape<ORDER>::GC < ca; ++bands) {
+        const Band b = band_from<ORDER>(g0, ca, nchunk, room, nsm);
+        if (b.ng < 1) return -1;
+        g0 += b.ng;
+    }
+    return bands;
+}
+
 template <int ORDER>
 cudaError_t launch_t(const ForceArgs &f, size_t cap, int nsm, cudaStream_t s, int *launches)
 {
@@ -25,23 +67,11 @@ cudaError_t launch_t(const ForceArgs &f, size_t cap, int nsm, cudaStream_t s, in
     const int groups = (a.ca + GC - 1) / GC;
     const long long chunk = F * 32, room = (long long)(cap / chunk);   // scratch in [F][32] blocks
     for (int g0 = 0; g0 < groups; g0 += a.ng) {
-        // as many groups as the scratch has rows and slice sums for, in slices
-        // that make 10 to 20 waves of CTAs, in whole tiles: 20 as long as the slice
-        // sums take no more than 0.4 of the rows' room (with 32 rows, 6th order, N =
-        // 131072: 4 waves 41.7 ms, 6 40.5, 10 40.0; with 64, 10 39.7, 20 39.3; N =
-        // 50000 5.92, 5.98)
+        const Band b = band_from<ORDER>(g0, a.ca, a.nchunk, room, nsm);
         a.g0 = g0;
-        a.ng = (int)std::min((long long)(groups - g0), room / a.ca);
-        for (int pass = 0; pass < 3; ++pass) {
-            if (a.ng < 1) return cudaErrorInvalidValue;
-            const long long units = (long long)a.ng * (a.nchunk - (long long)g0 * GC) - (long long)GC * a.ng * (a.ng - 1) / 2;
-            const long long wave = SymShape<ORDER>::MINB * nsm;
-            const long long lc = std::min(units / (10 * wave),
-                                          std::max(units / (20 * wave), 5LL * GC * a.nchunk / (2 * a.ca)));
-            a.lc = (int)std::max(1LL, (lc + kSymFTile - 1) / kSymFTile) * kSymFTile;
-            a.smax = sym_slices(a.nchunk, g0, GC, a.lc);
-            a.ng = (int)std::min((long long)a.ng, room / (a.ca + (long long)a.smax * GC));
-        }
+        a.ng = b.ng;
+        a.lc = b.lc;
+        a.smax = b.smax;
         if (a.ng < 1) return cudaErrorInvalidValue;
         a.rows = f.partial;
         a.cols = f.partial + (size_t)a.ng * a.ca * chunk;
@@ -72,6 +102,13 @@ bool force_sym_takes(int order, bool mixed, int nact, int npad, size_t cap)
     const size_t blocks = cap / (size_t)(3 * (order / 2) * 32);
     const bool most = nact >= 4096 && nact >= npad * 4LL / 10, many = nact >= 8192 && nact >= npad / 5;
     return (most || many) && blocks >= (size_t)npad / 32 * 2;
+}
+
+int force_sym_bands(int order, int nact, int npad, size_t cap, int nsm)
+{
+    if (!force_sym_takes(order, false, nact, npad, cap)) return 0;
+    const int ca = (nact + 31) / 32;
+    return order == 4 ? bands_t<4>(ca, npad / 32, cap, nsm) : bands_t<6>(ca, npad / 32, cap, nsm);
 }
 
 cudaError_t launch_force_sym(int order, const ForceArgs &f, size_t cap, int nsm, cudaStream_t s, int *launches)

@@ -178,6 +178,8 @@ cudaError_t launch_force_lanes(int order, const ForceArgs &a, int nsm, cudaStrea
 // FP64 force with every pair of active particles taken once (hb_force_sym.cuh);
 // needs f.pred and f.partial (cap doubles); *launches is advanced.
 bool force_sym_takes(int order, bool mixed, int nact, int npad, size_t cap);
+// Its launches of force_sym_kernel for that call: 0 when it is not taken.
+int force_sym_bands(int order, int nact, int npad, size_t cap, int nsm);
 cudaError_t launch_force_sym(int order, const ForceArgs &f, size_t cap, int nsm, cudaStream_t s,
                              int *launches);
 cudaError_t launch_predict(int order, bool mixed, const double *jp, int n, int npad,

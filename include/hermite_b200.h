@@ -168,6 +168,10 @@ int hb_force_variant_count(int order, int precision);
 /* Describe a variant: threads per CTA, i per thread, warps splitting j. */
 int hb_force_variant_info(int order, int precision, int variant,
                           int *threads, int *i_per_thread, int *j_warps);
+/* How many bands the force that takes each pair once (4th and 6th order, FP64,
+ * most particles active) is cut into for n particles, nact of them active, and
+ * a scratch of `doubles`, on a GPU of 148 SMs; 0: ordered pairs are taken. */
+int hb_force_pairs_once_bands(int order, int n, int nact, long long doubles);
 
 /* ---- device-resident block-step integration ------------------------------
  * The reference runs the Hermite corrector and the block-timestep scheduler
