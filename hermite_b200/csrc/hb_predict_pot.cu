@@ -120,7 +120,8 @@ cudaError_t launch_predict(int order, bool mixed, const double *jp, int n, int n
 // SRC/hermite4-titan.cu:303-327 and its 6th/8th-order counterparts).
 // A block takes 32 consecutive values and G groups of a warp each: group g adds slices
 // g, g + G, ... in 8 interleaved sums (8 loads in flight), combined pairwise;
-// the groups' sums are added in group order.
+// the groups' sums likewise: at most log2(G) + 2 roundings in a row there, where group
+// order had 31.
 template <int G>
 __global__ void __launch_bounds__(G * 32)
 reduce_kernel(const double *__restrict__ partial, size_t stride, int S, int v,
@@ -144,10 +145,19 @@ reduce_kernel(const double *__restrict__ partial, size_t stride, int S, int v,
     red[g][lane] = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
     __syncthreads();
     if (g == 0 && e < v) {
-        double sum = red[0][lane];
+        constexpr int W = G < 8 ? G : 8;
+        double sum[W];
 #pragma unroll
-        for (int k = 1; k < G; ++k) sum += red[k][lane];
-        force[e] = sum;
+        for (int u = 0; u < W; ++u) {
+            sum[u] = red[u][lane];
+#pragma unroll
+            for (int k = u + W; k < G; k += W) sum[u] += red[k][lane];
+        }
+#pragma unroll
+        for (int w = W / 2; w > 0; w /= 2)
+#pragma unroll
+            for (int u = 0; u < w; ++u) sum[u] += sum[u + w];
+        force[e] = sum[0];
     }
 }
 
