@@ -5,6 +5,7 @@
 #include <climits>
 #include <cmath>
 #include <cstdarg>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -62,10 +63,13 @@ struct hb_ctx {
     double *h_force_dev = nullptr;  // device address of the mapped h_force
     double *d_jp = nullptr, *d_force = nullptr, *d_pot = nullptr, *d_posm = nullptr;
     double *d_partial = nullptr;
+    double *d_rows = nullptr;       // larger scratch of the each-pair-once force (rows_scratch)
     void *d_pred = nullptr;
     unsigned *d_counter = nullptr;
     int *h_err = nullptr, *d_err = nullptr;
     size_t partial_cap = 0;         // doubles
+    size_t rows_cap = 0;
+    bool rows_tried = false;
 
     std::atomic<int> dirty_lo{INT_MAX}, dirty_hi{0};
     std::atomic<bool> upload_pending{false};
@@ -308,6 +312,29 @@ int pick_variant(const hb_ctx *c, int nact, int *jsplit_hint)
 // mapped pinned buffer (no device->host copy in the block step).
 constexpr size_t kZeroCopyBytes = 256 << 10;
 
+// The scratch of the each-pair-once force: rows of a force record per slot, 64 of
+// them up to 512 MiB, made by the first call of at least 2^30 pairs, since contexts
+// that never move most of a large system have no use for it.  Smaller calls, a
+// capture, which may not allocate, and a full memory use the slices' buffer.  6th
+// order, all active, that buffer against this scratch: N = 20000 1.12 / 1.08 ms, 32768
+// 2.88 / 2.66, 65536 12.4 / 10.9, 131072 (32 rows up to 256 MiB) 40.0 / 39.3.  Making
+// it took 0 to 4 ms.
+constexpr long long kRowsPairs = 1LL << 30;
+
+void rows_scratch(hb_ctx *c, int nact)
+{
+    if (c->rows_tried || (long long)nact * c->npad < kRowsPairs) return;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return;
+    c->rows_tried = true;
+    const size_t want = std::min((size_t)64 * c->npad * c->F, (size_t)64 << 20);
+    if (want <= c->partial_cap) return;
+    if (cudaMalloc((void **)&c->d_rows, want * sizeof(double)) == cudaSuccess)
+        c->rows_cap = want;
+    else
+        (void)cudaGetLastError();
+}
+
 int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
 {
     if (nact == 0) return HB_OK;
@@ -331,8 +358,11 @@ int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
         return HB_OK;
     }
     const bool automatic = ctx->variant_override < 0 && ctx->jsplit_override == 0;
-    if (automatic && force_out_dev == ctx->d_force &&
-        force_sym_takes(ctx->order, mixed, nact, ctx->npad, ctx->partial_cap)) {
+    const bool most = automatic && force_out_dev == ctx->d_force &&
+                      force_sym_takes(ctx->order, mixed, nact, ctx->npad, SIZE_MAX);
+    if (most) rows_scratch(ctx, nact);
+    const size_t cap = std::max(ctx->rows_cap, ctx->partial_cap);
+    if (most && force_sym_takes(ctx->order, mixed, nact, ctx->npad, cap)) {
         // most particles move: every pair once
         if (ctx->pred_stale) {
             HB_CK(launch_predict(ctx->order, mixed, ctx->d_jp, ctx->nbody, ctx->npad, ctx->tsys,
@@ -346,11 +376,11 @@ int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
         a.nact = nact;
         a.eps2 = eps2;
         a.force = force_out_dev;
-        a.partial = ctx->d_partial;
+        a.partial = ctx->rows_cap ? ctx->d_rows : ctx->d_partial;
         a.err = ctx->d_err;
         a.spin = ctx->wait_limit;
         int launches = 0;
-        HB_CK(launch_force_sym(ctx->order, a, ctx->partial_cap, ctx->nsm, ctx->stream, &launches));
+        HB_CK(launch_force_sym(ctx->order, a, cap, ctx->nsm, ctx->stream, &launches));
         ctx->launches += launches;
         return HB_OK;
     }
@@ -469,6 +499,7 @@ int hb_destroy(hb_ctx *ctx)
     cudaFree(ctx->d_pot);
     cudaFree(ctx->d_posm);
     cudaFree(ctx->d_partial);
+    cudaFree(ctx->d_rows);
     cudaFree(ctx->d_pred);
     cudaFree(ctx->d_counter);
     if (ctx->int_exec) cudaGraphExecDestroy(ctx->int_exec);
@@ -526,13 +557,9 @@ int hb_create(int order, int nbody, int precision, hb_ctx **out)
     const size_t np = ctx->npad;
     const size_t pred_bytes = std::max(np * pred64_ncomp(order) * sizeof(double),
                                        np * predmx_ncomp(order) * sizeof(float));
-    // j-slices' partials; or rows of one double per value and slot for pairs
-    // taken once: 64 rows up to 512 MiB (32 rows up to 256 MiB: 3-7 % slower at N =
-    // 20000 ... 65536, 1 % at 131072), and 64 MiB from 4096 slots on, which
-    // takes 8192 in one launch (0.124 ms at 4th order; in two, 0.153)
-    const size_t slices_cap = (size_t)2 * ctx->nsm * 8 * 256 * ctx->F;
-    ctx->partial_cap = std::max(slices_cap, std::min(64 * np * ctx->F, (size_t)64 << 20));
-    if (np >= 4096) ctx->partial_cap = std::max(ctx->partial_cap, (size_t)8 << 20);
+    // j-slices' partials, and the rows of small each-pair-once calls (all of 8192 in
+    // one launch)
+    ctx->partial_cap = (size_t)2 * ctx->nsm * 10 * 256 * ctx->F;
     bool ok = true;
     ok = ok && cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&ctx->ev_upload, cudaEventDisableTiming) == cudaSuccess;
@@ -547,12 +574,7 @@ int hb_create(int order, int nbody, int precision, hb_ctx **out)
     ok = ok && cudaMalloc((void **)&ctx->d_posm, np * (order == 9 ? 7 : 4) * sizeof(double)) == cudaSuccess;
     ok = ok && cudaMalloc(&ctx->d_pred, pred_bytes) == cudaSuccess;
     ok = ok && cudaMalloc((void **)&ctx->d_counter, (np / 32 + 1) * sizeof(unsigned)) == cudaSuccess;
-    if (ok && cudaMalloc((void **)&ctx->d_partial, ctx->partial_cap * sizeof(double)) != cudaSuccess) {
-        // little memory left: room for the slices only (fewer rows, or ordered pairs)
-        (void)cudaGetLastError();
-        ctx->partial_cap = slices_cap;
-        ok = cudaMalloc((void **)&ctx->d_partial, ctx->partial_cap * sizeof(double)) == cudaSuccess;
-    }
+    ok = ok && cudaMalloc((void **)&ctx->d_partial, ctx->partial_cap * sizeof(double)) == cudaSuccess;
     if (ok) {
         ok = cudaHostGetDevicePointer((void **)&ctx->d_err, ctx->h_err, 0) == cudaSuccess &&
              cudaHostGetDevicePointer((void **)&ctx->h_force_dev, ctx->h_force, 0) == cudaSuccess;

@@ -21,6 +21,7 @@ EPS2 = (1.0 / 256) ** 2
     (4, 16384, 16384), (6, 12289, 12000),
     (4, 15000, 6001), (6, 15000, 6001),      # the smallest active part, ragged
     (4, 40900, 8193), (6, 40900, 8193),      # and of a large system
+    (4, 32897, 32897),                       # with the larger scratch
 ])
 def test_pairs_once_against_oracle(order, n, nact, oracle):
     rec = make_records(order, n, seed=71)

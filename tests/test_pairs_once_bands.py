@@ -1,12 +1,12 @@
 """The each-pair-once force finds bands of groups for every scratch it is taken
-with: the smallest the library falls back to where little GPU memory is left
-(the j-slices' partial sums, 2 x 148 x 8 x 256 force records), just enough for
-two rows, and the usual one (CPU)."""
+with: the j-slices' partial sums (2 x 148 x 10 x 256 force records), which smaller
+calls use and larger ones where little GPU memory is left, just enough for two
+rows, and 512 MiB (CPU)."""
 import pytest
 
 import hermite_b200 as hb
 
-SLICES = 2 * 148 * 8 * 256          # force records
+SLICES = 2 * 148 * 10 * 256         # force records
 
 
 @pytest.mark.parametrize("order", [4, 6])
