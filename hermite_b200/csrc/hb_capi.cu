@@ -63,7 +63,7 @@ struct hb_ctx {
     double *h_force_dev = nullptr;  // device address of the mapped h_force
     double *d_jp = nullptr, *d_force = nullptr, *d_pot = nullptr, *d_posm = nullptr;
     double *d_partial = nullptr;
-    double *d_rows = nullptr;       // larger scratch of the each-pair-once force (rows_scratch)
+    double *d_rows = nullptr;       // larger scratch of the each-pair-once force (pairs_once_scratch)
     void *d_pred = nullptr;
     unsigned *d_counter = nullptr;
     int *h_err = nullptr, *d_err = nullptr;
@@ -312,27 +312,40 @@ int pick_variant(const hb_ctx *c, int nact, int *jsplit_hint)
 // mapped pinned buffer (no device->host copy in the block step).
 constexpr size_t kZeroCopyBytes = 256 << 10;
 
-// The scratch of the each-pair-once force: rows of a force record per slot, 64 of
-// them up to 512 MiB, made by the first call of at least 2^30 pairs, since contexts
-// that never move most of a large system have no use for it.  Smaller calls, a
-// capture, which may not allocate, and a full memory use the slices' buffer.  6th
-// order, all active, that buffer against this scratch: N = 20000 1.12 / 1.08 ms, 32768
-// 2.88 / 2.66, 65536 12.4 / 10.9, 131072 (32 rows up to 256 MiB) 40.0 / 39.3.  Making
-// it took 0 to 4 ms.
+// The scratch of the each-pair-once force for calls of at least 2^30 pairs: rows of
+// a force record per slot, 64 of them up to 512 MiB, made by the first such call,
+// since contexts that never move most of a large system have no use for it.  Smaller
+// calls use the slices' buffer, before and after it is made alike: the scratch sets
+// the bands, hence the association of the sums, and a call's bits may not depend on
+// the calls before it.  Large calls use that buffer too, all of them, when the memory
+// is full, and those in a capture before the first other one, which may not allocate.
+// 6th order, all active, that buffer against this scratch: N = 20000 1.12 / 1.08
+// ms, 32768 2.88 / 2.66, 65536 12.4 / 10.9, 131072 (32 rows up to 256 MiB) 40.0 /
+// 39.3.  Making it took 0 to 4 ms.
 constexpr long long kRowsPairs = 1LL << 30;
 
-void rows_scratch(hb_ctx *c, int nact)
+struct Scratch {
+    double *p;
+    size_t cap;      // doubles
+};
+
+Scratch pairs_once_scratch(hb_ctx *c, int nact)
 {
-    if (c->rows_tried || (long long)nact * c->npad < kRowsPairs) return;
+    const Scratch small{c->d_partial, c->partial_cap};
+    if ((long long)nact * c->npad < kRowsPairs) return small;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return;
-    c->rows_tried = true;
-    const size_t want = std::min((size_t)64 * c->npad * c->F, (size_t)64 << 20);
-    if (want <= c->partial_cap) return;
-    if (cudaMalloc((void **)&c->d_rows, want * sizeof(double)) == cudaSuccess)
-        c->rows_cap = want;
-    else
-        (void)cudaGetLastError();
+    if (!c->rows_tried && cudaStreamIsCapturing(c->stream, &st) == cudaSuccess &&
+        st == cudaStreamCaptureStatusNone) {
+        c->rows_tried = true;
+        const size_t want = std::min((size_t)64 * c->npad * c->F, (size_t)64 << 20);
+        if (want > c->partial_cap) {
+            if (cudaMalloc((void **)&c->d_rows, want * sizeof(double)) == cudaSuccess)
+                c->rows_cap = want;
+            else
+                (void)cudaGetLastError();
+        }
+    }
+    return c->rows_cap ? Scratch{c->d_rows, c->rows_cap} : small;
 }
 
 int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
@@ -360,9 +373,8 @@ int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
     const bool automatic = ctx->variant_override < 0 && ctx->jsplit_override == 0;
     const bool most = automatic && force_out_dev == ctx->d_force &&
                       force_sym_takes(ctx->order, mixed, nact, ctx->npad, SIZE_MAX);
-    if (most) rows_scratch(ctx, nact);
-    const size_t cap = std::max(ctx->rows_cap, ctx->partial_cap);
-    if (most && force_sym_takes(ctx->order, mixed, nact, ctx->npad, cap)) {
+    const Scratch scratch = most ? pairs_once_scratch(ctx, nact) : Scratch{};
+    if (most && force_sym_takes(ctx->order, mixed, nact, ctx->npad, scratch.cap)) {
         // most particles move: every pair once
         if (ctx->pred_stale) {
             HB_CK(launch_predict(ctx->order, mixed, ctx->d_jp, ctx->nbody, ctx->npad, ctx->tsys,
@@ -376,11 +388,11 @@ int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
         a.nact = nact;
         a.eps2 = eps2;
         a.force = force_out_dev;
-        a.partial = ctx->rows_cap ? ctx->d_rows : ctx->d_partial;
+        a.partial = scratch.p;
         a.err = ctx->d_err;
         a.spin = ctx->wait_limit;
         int launches = 0;
-        HB_CK(launch_force_sym(ctx->order, a, cap, ctx->nsm, ctx->stream, &launches));
+        HB_CK(launch_force_sym(ctx->order, a, scratch.cap, ctx->nsm, ctx->stream, &launches));
         ctx->launches += launches;
         return HB_OK;
     }
