@@ -905,8 +905,6 @@ int setup_integrator(hb_ctx *ctx, double tsys, double eps2, double eta, double d
     ctx->h_status->particle_steps = particle_steps;
     ctx->h_status->block_steps = block_steps;
     HB_CK(cudaMemcpy(ctx->d_sched, &sc, sizeof(Sched), cudaMemcpyHostToDevice));
-    const TeamSys ts{0, ctx->nbody, 0, eps2};
-    HB_CK(cudaMemcpy(ctx->d_team_sys, &ts, sizeof(TeamSys), cudaMemcpyHostToDevice));
 
     IntegratorLaunch L{};
     L.jp = ctx->d_jp;
@@ -1109,7 +1107,10 @@ int run_team(hb_ctx *ctx, const TeamConfig &cfg, double tend, long long max_bloc
 {
     volatile IntStatus *st = ctx->h_status;
     HB_CK(team_sched_sync(ctx->d_sched, ctx->d_team_state, true, ctx->stream));
-    TeamLaunch L;
+    TeamSys sys{};
+    sys.n = ctx->nbody;
+    sys.eps2 = ctx->h_sched->eps2;
+    TeamLaunch L{};
     L.jp = ctx->d_jp;
     L.dt = ctx->d_dt;
     L.aux = ctx->d_aux;
@@ -1119,6 +1120,8 @@ int run_team(hb_ctx *ctx, const TeamConfig &cfg, double tend, long long max_bloc
     L.nsys = 1;
     if (team_shape(ctx->order, cfg, ctx->nbody, &L) != 0)
         return fail(ctx, HB_ERR_TOO_LARGE, "the system does not fit a team of %d CTAs", cfg.ctas);
+    sys.im = L.im;
+    HB_CK(cudaMemcpyAsync(ctx->d_team_sys, &sys, sizeof(TeamSys), cudaMemcpyHostToDevice, ctx->stream));
     L.tend = tend;
     L.etapow = ctx->h_sched->etapow;
     L.dtmax = ctx->h_sched->dtmax;

@@ -44,8 +44,8 @@ struct Cluster {
     double eps2;
 };
 
-// Clusters integrated by team kernels of one size: systems [first,
-// first + count) of the team system table.
+// Clusters integrated by team kernels of one size and one place of the records:
+// systems [first, first + count) of the team system table.
 struct TeamGroup {
     int ctas, first, count, nmax;
     TeamConfig cfg;
@@ -652,7 +652,7 @@ struct hb_ens {
     EnsTotals *h_tot = nullptr, *d_tot = nullptr;   // mapped
     TeamSys *d_tsys = nullptr;                      // team systems, grouped by team size
     int *d_tidx = nullptr;                          // their cluster indices
-    int *d_team_next = nullptr;                     // one queue head per team size
+    int *d_team_next = nullptr;                     // one queue head per group
     cudaEvent_t ev_fork = nullptr;                  // team groups beside one another
     std::vector<cudaStream_t> team_streams;
     std::vector<cudaEvent_t> team_events;
@@ -756,22 +756,26 @@ int build_groups(hb_ens *e)
         std::vector<int> &v = by[C];
         // largest systems first: the queue's tail is short
         std::stable_sort(v.begin(), v.end(), [&](int a, int b) { return e->cl[a].n > e->cl[b].n; });
-        TeamGroup g;
-        g.ctas = C;
-        g.first = (int)ts.size();
-        g.count = (int)v.size();
-        g.nmax = e->cl[v.front()].n;
-        g.cfg = cfgs[C];
-        for (int c : v) {
-            TeamSys t;
-            t.off = e->cl[c].off;
-            t.n = e->cl[c].n;
-            t.id = c;
-            t.eps2 = e->cl[c].eps2;
-            ts.push_back(t);
-            idx.push_back(c);
+        for (const bool rsmem : {true, false}) {
+            TeamGroup g{C, (int)ts.size(), 0, 0, cfgs[C]};
+            for (int c : v) {
+                TeamLaunch alone{};
+                if (team_shape(e->order, cfgs[C], e->cl[c].n, &alone) != 0)
+                    return ens_fail(e, HB_ERR_TOO_LARGE, "a cluster does not fit its team");
+                if (alone.rsmem != rsmem) continue;
+                TeamSys t;
+                t.off = e->cl[c].off;
+                t.n = e->cl[c].n;
+                t.id = c;
+                t.im = alone.im;
+                t.eps2 = e->cl[c].eps2;
+                ts.push_back(t);
+                idx.push_back(c);
+                g.nmax = std::max(g.nmax, t.n);
+                ++g.count;
+            }
+            if (g.count) e->groups.push_back(g);
         }
-        e->groups.push_back(g);
     }
     if (!ts.empty()) {
         cudaError_t ce = cudaMemcpy(e->d_tsys, ts.data(), ts.size() * sizeof(TeamSys), cudaMemcpyHostToDevice);
@@ -792,7 +796,7 @@ int totals(hb_ens *e, const int *idx, int count)
     return ce == cudaSuccess ? HB_OK : ens_fail(e, HB_ERR_CUDA, "cluster totals", ce);
 }
 
-// Every team-engine cluster integrated to tend.  The groups (one per team size)
+// Every team-engine cluster integrated to tend.  The groups (by team size)
 // run beside one another, each on its own stream, the largest teams first: one
 // after the other, each group leaves most of the GPU idle (32 clusters of 256 ...
 // 4096 particles, 4th order, teams of powers of two: 43.0 against 18.7 ms).
@@ -981,7 +985,7 @@ int hb_ens_create(int order, int nclusters, const int *sizes, int precision, hb_
               cudaHostGetDevicePointer((void **)&e->d_tot, e->h_tot, 0) == cudaSuccess &&
               cudaMalloc((void **)&e->d_tsys, nclusters * sizeof(TeamSys)) == cudaSuccess &&
               cudaMalloc((void **)&e->d_tidx, nclusters * sizeof(int)) == cudaSuccess &&
-              cudaMalloc((void **)&e->d_team_next, 16 * sizeof(int)) == cudaSuccess;
+              cudaMalloc((void **)&e->d_team_next, 32 * sizeof(int)) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         hb_ens_destroy(e);

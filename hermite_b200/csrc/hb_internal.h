@@ -124,6 +124,7 @@ struct TeamSys {
     long long off;     // first slot of the system in the record / dt arrays
     int n;
     int id;            // index of the system's TeamState
+    int im;            // i-states per round in a launch of its own (team_shape)
     double eps2;
 };
 struct TeamState {     // per system, persistent across launches
@@ -152,8 +153,9 @@ struct TeamLaunch {
     long long max_steps;   // per system and launch
 };
 cudaError_t team_setup(int order, int ctas, TeamConfig *cfg);
-// Fills L's ctas, jl_cap, im and smem for systems of up to nmax particles;
-// -1 when they do not fit a team of cfg.ctas CTAs.
+// Fills L's ctas, jl_cap, im, smem and rsmem for systems of up to nmax particles;
+// -1 when they do not fit a team of cfg.ctas CTAs.  A launch takes systems whose
+// own rsmem is alike.
 int team_shape(int order, const TeamConfig &cfg, int nmax, TeamLaunch *L);
 cudaError_t team_launch(int order, const TeamLaunch &L, int teams, cudaStream_t s);
 cudaError_t team_sched_sync(Sched *s, TeamState *st, bool to_team, cudaStream_t stream);

@@ -94,18 +94,18 @@ __device__ __forceinline__ double warp_min(double v)
 }
 
 // Partial forces of nr i-particles (ibuf, AoSoA32, at positions idx(gi))
-// against this CTA's JL own predicted slots.  G lanes (a power of two)
-// share NI i-particles, each lane summing every G-th own slot, and their
-// sums meet in a fixed xor-shuffle tree; out(idx, f) is called by the first
-// lane of each group.
+// against this CTA's JL own predicted slots.  G lanes (a power of two, wide enough
+// for ng of them at once where that goes) share NI i-particles, each lane summing
+// every G-th own slot, and their sums meet in a fixed xor-shuffle tree; out(idx,
+// f) is called by the first lane of each group.
 template <int ORDER, int NI, typename Idx, typename Out>
 __device__ __forceinline__ void team_force_ni(const double *ibuf, const double *pred, int JL, int nr,
-                                              double eps2, Idx idx, Out out)
+                                              int ng, double eps2, Idx idx, Out out)
 {
     constexpr int NW = kTeamWarps, F = Frc<ORDER>::words;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int G = 32;
-    while (G > 1 && NW * (32 / G) * NI < nr) G >>= 1;
+    while (G > 1 && NW * (32 / G) * NI < ng) G >>= 1;
     const int js = lane & (G - 1), slots = NW * (32 / G);
     // more than a pair of i per thread: in rounds
     for (int g0 = 0; g0 * NI < nr; g0 += slots) {
@@ -145,19 +145,19 @@ __device__ __forceinline__ void team_force_ni(const double *ibuf, const double *
 
 // Two i per lane (two independent chains per j load) at 4th order, where the
 // registers allow it, once the round is large enough for the lane groups to
-// stay narrow; one otherwise.  The choice depends on nr only, so every CTA
-// of a team sums in the same order.
+// stay narrow; one otherwise.  The choice, like G, depends on ng only, so every
+// CTA of a team sums in the same order.
 template <int ORDER, typename Idx, typename Out>
 __device__ __forceinline__ void team_force(const double *ibuf, const double *pred, int JL, int nr,
-                                           double eps2, Idx idx, Out out)
+                                           int ng, double eps2, Idx idx, Out out)
 {
     if constexpr (ORDER == 4) {
-        if (nr > 128) {
-            team_force_ni<ORDER, 2>(ibuf, pred, JL, nr, eps2, idx, out);
+        if (ng > 128) {
+            team_force_ni<ORDER, 2>(ibuf, pred, JL, nr, ng, eps2, idx, out);
             return;
         }
     }
-    team_force_ni<ORDER, 1>(ibuf, pred, JL, nr, eps2, idx, out);
+    team_force_ni<ORDER, 1>(ibuf, pred, JL, nr, ng, eps2, idx, out);
 }
 
 template <int ORDER, bool RSMEM>
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
     int *gq = cand + jl_cap;                                      // [IM]
     int *gc = gq + IM;                                            // [IM]
     int *koff = gc + IM;                                          // [48] koff[c] = actives below rank c
-    int *misc = koff + 48;                                        // [0] system (rank 0), [1] own error
+    int *misc = koff + 48;                                        // [0] system (rank 0), [1] own error, [2] S.im
     __shared__ TeamXch own_xch;                                   // this rank's (m, k, err)
     TeamXch *own = &own_xch;
 
@@ -225,7 +225,10 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
                 tn[q] = inf;
             }
         }
-        if (tid == 0) misc[1] = 0;
+        if (tid == 0) {
+            misc[1] = 0;
+            misc[2] = S.im;
+        }
         double tsys = L.st[S.id].tsys;
         const bool dead = L.st[S.id].error != 0;   // a system that failed stays stopped
         long long steps = 0, psteps = 0;
@@ -349,7 +352,7 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
                 // sits at ibuf[c * KM + a]; partials go to the owner's part
                 // at [rank * KM + a]
                 team_force<ORDER>(
-                    ibuf, pred, JL, nact, eps2,
+                    ibuf, pred, JL, nact, nact, eps2,
                     [&](int gi) {
                         // koff is ascending: the last rank with koff[c] <= gi
                         int c = 0;
@@ -394,10 +397,16 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
                 __syncthreads();
                 announce();
             } else {
-                // many actives: rounds of IM pulled from the owners
+                // many actives: rounds pulled from the owners.  The lanes per
+                // i-particle are chosen from the rounds of misc[2] that the system has
+                // when it is alone in a launch; IM, which comes from the largest
+                // system of this one, only cuts those in parts.  So a system's sums,
+                // here and above, do not depend on the others (IM is above misc[2]
+                // only where that holds every slot).
                 team.sync();   // barrier 2: predicted states and candidate lists complete
-                for (int base = 0; base < nact; base += IM) {
-                    const int nr = min(IM, nact - base);
+                for (int r0 = 0; r0 < nact; r0 += misc[2])
+                for (int base = r0; base < min(r0 + misc[2], nact); base += IM) {
+                    const int nr = min(IM, min(r0 + misc[2], nact) - base), ng = min(misc[2], nact - r0);
                     for (int i = tid; i < nr; i += T) {
                         const int g = base + i;
                         int c = 0;
@@ -413,7 +422,7 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
                     }
                     __syncthreads();
                     team_force<ORDER>(
-                        ibuf, pred, JL, nr, eps2, [](int gi) { return gi; },
+                        ibuf, pred, JL, nr, ng, eps2, [](int gi) { return gi; },
                         [&](int gi, const double *f) {
 #pragma unroll
                             for (int k = 0; k < F; ++k) part[gi * F + k] = f[k];
@@ -440,7 +449,7 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
                         dts[q] = dtn;
                         tn[q] = dtn + r[7];
                     }
-                    if (base + IM < nact) team.sync();   // part and ibuf are reused by the next round
+                    if (base + nr < nact) team.sync();   // part and ibuf are reused by the next round
                 }
                 __syncthreads();
                 if (w == 0) find_candidates();
