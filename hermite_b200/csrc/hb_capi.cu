@@ -309,7 +309,9 @@ int pick_variant(const hb_ctx *c, int nact, int *jsplit_hint)
 }
 
 // Force records up to this size are written by the kernel straight into the
-// mapped pinned buffer (no device->host copy in the block step).
+// mapped pinned buffer (no device->host copy in the block step).  The each-pair-once
+// force, whose bands keep their running sums on the device, starts above it
+// (force_sym_takes), so which kernel runs does not depend on where the results go.
 constexpr size_t kZeroCopyBytes = 256 << 10;
 
 // The scratch of the each-pair-once force for calls of at least 2^30 pairs: rows of
@@ -371,7 +373,7 @@ int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
         return HB_OK;
     }
     const bool automatic = ctx->variant_override < 0 && ctx->jsplit_override == 0;
-    const bool most = automatic && force_out_dev == ctx->d_force &&
+    const bool most = automatic &&
                       force_sym_takes(ctx->order, mixed, nact, ctx->npad, SIZE_MAX);
     const Scratch scratch = most ? pairs_once_scratch(ctx, nact) : Scratch{};
     if (most && force_sym_takes(ctx->order, mixed, nact, ctx->npad, scratch.cap)) {

@@ -91,16 +91,21 @@ cudaError_t launch_t(const ForceArgs &f, size_t cap, int nsm, cudaStream_t s, in
 
 // The share of the pairs that is one-sided grows as fewer particles are active, and
 // small calls do not fill the waves.  Both sides measured (ms, ordered pairs /
-// pairs once): all of N = 4096 0.060 / 0.049 at 4th order and 0.088 / 0.090 at
-// 6th, 131072 59.9 / 39.0 (6th); a fifth of N = 40000 0.656 / 0.640 (4th) and
-// 1.122 / 1.090 (6th), of 262144 47.1 / 44.0 (6th), 0.15 of 65536 1.291 / 1.302
-// (4th); 4096 of 16384 0.155 / 0.157 (4th) and 0.252 / 0.259 (6th).  The 8th-order
-// sums are compensated; they keep ordered pairs.
+// pairs once): all of N = 4096 0.088 / 0.090 at 6th order, 131072 59.9 / 39.0
+// (6th); a fifth of N = 40000 0.656 / 0.640 (4th) and 1.122 / 1.090 (6th), of
+// 262144 47.1 / 44.0 (6th), 0.15 of 65536 1.291 / 1.302 (4th); 4096 of 16384 0.252 /
+// 0.259 (6th).  At 4th order it starts where the results are too large to be
+// written straight to the host (kZeroCopyBytes, hb_capi.cu: 5461 records): below,
+// whole calls through the host take longer with it and the copy that the bands'
+// device sums then need (4096 of 4500 106 / 121 us, of 8000 133 / 141, 4800 of 8000 158 /
+// 161), and one rule has to serve every entry point, or their bits would differ.
+// The 8th-order sums are compensated; they keep ordered pairs.
 bool force_sym_takes(int order, bool mixed, int nact, int npad, size_t cap)
 {
     if (mixed || (order != 4 && order != 6)) return false;
     const size_t blocks = cap / (size_t)(3 * (order / 2) * 32);
-    const bool most = nact >= 4096 && nact >= npad * 4LL / 10, many = nact >= 8192 && nact >= npad / 5;
+    const bool most = nact >= (order == 4 ? 5462 : 4096) && nact >= npad * 4LL / 10;
+    const bool many = nact >= 8192 && nact >= npad / 5;
     return (most || many) && blocks >= (size_t)npad / 32 * 2;
 }
 
