@@ -875,7 +875,7 @@ int integrator_alloc(hb_ctx *ctx)
               cudaMalloc((void **)&ctx->d_team_state, sizeof(TeamState)) == cudaSuccess &&
               cudaMalloc((void **)&ctx->d_team_next, sizeof(int)) == cudaSuccess &&
               cudaMalloc((void **)&ctx->d_gbar, 2 * sizeof(unsigned)) == cudaSuccess &&
-              cudaMemset(ctx->d_gbar, 0, 2 * sizeof(unsigned)) == cudaSuccess;
+              cudaMemsetAsync(ctx->d_gbar, 0, 2 * sizeof(unsigned), ctx->stream) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         return fail(ctx, HB_ERR_ALLOC, "integrator buffers could not be allocated");
@@ -906,7 +906,9 @@ int setup_integrator(hb_ctx *ctx, double tsys, double eps2, double eta, double d
     ctx->h_status->tsys = tsys;
     ctx->h_status->particle_steps = particle_steps;
     ctx->h_status->block_steps = block_steps;
-    HB_CK(cudaMemcpy(ctx->d_sched, &sc, sizeof(Sched), cudaMemcpyHostToDevice));
+    // on the stream, like every upload here: a plain copy from pageable memory may
+    // return with its last part under way, and the stream would not wait for it
+    HB_CK(cudaMemcpyAsync(ctx->d_sched, &sc, sizeof(Sched), cudaMemcpyHostToDevice, ctx->stream));
 
     IntegratorLaunch L{};
     L.jp = ctx->d_jp;
@@ -1223,7 +1225,7 @@ int hb_integrator_run(hb_ctx *ctx, double tend, long long max_block_steps)
     if (s != HB_OK) return s;
     volatile IntStatus *st = ctx->h_status;
     if (!(tend >= st->tsys)) return fail(ctx, HB_ERR_INVALID, "tend %g is before tsys %g", tend, st->tsys);
-    HB_CK(cudaMemcpy(&ctx->d_sched->tend, &tend, sizeof(double), cudaMemcpyHostToDevice));
+    HB_CK(cudaMemcpyAsync(&ctx->d_sched->tend, &tend, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     TeamConfig cfg{};
     const int engine = resolve_engine(ctx, &cfg);
     if (engine < 0) return -engine;

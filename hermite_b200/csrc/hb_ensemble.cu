@@ -677,6 +677,15 @@ int ens_fail(hb_ens *e, int status, const char *msg, cudaError_t ce = cudaSucces
     return status;
 }
 
+// Every upload goes on the ensemble's stream, before the kernels that read it.  A
+// plain cudaMemcpy from pageable memory may return with its last part under way, and
+// the stream, a non-blocking one, would not wait for it.  (The source is read
+// before the call returns, so it may be a local.)
+cudaError_t upload(hb_ens *e, void *dst, const void *src, size_t bytes)
+{
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, e->stream);
+}
+
 // Team size for a cluster of n particles: a CTA per kEnsTeamSlots, more if its
 // slots do not fit the CTAs' shared memory; a function of n alone, so that a
 // cluster's sums do not depend on the other clusters.  Smaller teams use the
@@ -778,9 +787,8 @@ int build_groups(hb_ens *e)
         }
     }
     if (!ts.empty()) {
-        cudaError_t ce = cudaMemcpy(e->d_tsys, ts.data(), ts.size() * sizeof(TeamSys), cudaMemcpyHostToDevice);
-        if (ce == cudaSuccess)
-            ce = cudaMemcpy(e->d_tidx, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice);
+        cudaError_t ce = upload(e, e->d_tsys, ts.data(), ts.size() * sizeof(TeamSys));
+        if (ce == cudaSuccess) ce = upload(e, e->d_tidx, idx.data(), idx.size() * sizeof(int));
         if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "team system table", ce);
     }
     e->groups_ready = true;
@@ -1002,11 +1010,11 @@ int hb_ens_create(int order, int nclusters, const int *sizes, int precision, hb_
     std::vector<double> dt(ns, INFINITY);
     for (size_t i = 0; i < ns; ++i)
         for (int k = 0; k < 3; ++k) pad[i * e->R + k] = 1099511627776.0 + (double)(i * 3 + k);
-    ok = cudaMemcpy(e->d_jp, pad.data(), pad.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess &&
-         cudaMemcpy(e->d_dt, dt.data(), dt.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess &&
-         cudaMemcpy(e->d_slot_cluster, slot_cluster.data(), slot_cluster.size() * sizeof(int),
-                    cudaMemcpyHostToDevice) == cudaSuccess &&
-         cudaMemset(e->d_counter, 0, (ns / 32 + nclusters + 1) * sizeof(unsigned)) == cudaSuccess;
+    ok = upload(e, e->d_jp, pad.data(), pad.size() * sizeof(double)) == cudaSuccess &&
+         upload(e, e->d_dt, dt.data(), dt.size() * sizeof(double)) == cudaSuccess &&
+         upload(e, e->d_slot_cluster, slot_cluster.data(), slot_cluster.size() * sizeof(int)) == cudaSuccess &&
+         cudaMemsetAsync(e->d_counter, 0, (ns / 32 + nclusters + 1) * sizeof(unsigned), e->stream) == cudaSuccess &&
+         cudaStreamSynchronize(e->stream) == cudaSuccess;
     if (!ok) {
         hb_ens_destroy(e);
         return HB_ERR_CUDA;
@@ -1122,7 +1130,7 @@ int hb_ens_init(hb_ens *e, double tsys, double eta, double eta_s, double dtmax)
     if (e->exec) { cudaGraphExecDestroy(e->exec); e->exec = nullptr; }
     if (e->graph) { cudaGraphDestroy(e->graph); e->graph = nullptr; }
     e->ready = false;
-    ce = cudaMemcpy(e->d_cl, e->cl.data(), e->cl.size() * sizeof(Cluster), cudaMemcpyHostToDevice);
+    ce = upload(e, e->d_cl, e->cl.data(), e->cl.size() * sizeof(Cluster));
     if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "cluster table", ce);
     // tlast = tsys, derivatives zero, for every real slot
     ens_reset_kernel<<<e->nslot / kClusterPad, kClusterPad, 0, e->stream>>>(e->d_jp, e->R, e->d_cl,
@@ -1138,7 +1146,7 @@ int hb_ens_init(hb_ens *e, double tsys, double eta, double eta_s, double dtmax)
     s.etapow = std::pow(eta, 2.0 * (e->order - 3));
     s.dtmax = dtmax;
     s.status = e->d_st;
-    ce = cudaMemcpy(e->d_s, &s, sizeof(EnsSched), cudaMemcpyHostToDevice);
+    ce = upload(e, e->d_s, &s, sizeof(EnsSched));
     if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "scheduler upload", ce);
     const bool m = e->precision == HB_MIXED;
     const int passes = e->order > 4 ? 2 : 1;
@@ -1157,7 +1165,7 @@ int hb_ens_init(hb_ens *e, double tsys, double eta, double eta_s, double dtmax)
     s.interactions = 0.0;
     s.tnext_bits = kInf;
     s.tsys = tsys;
-    ce = cudaMemcpy(e->d_s, &s, sizeof(EnsSched), cudaMemcpyHostToDevice);
+    ce = upload(e, e->d_s, &s, sizeof(EnsSched));
     if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "scheduler upload", ce);
     std::memset(e->h_st, 0, sizeof(EnsStatus));
     e->h_st->tsys = tsys;
@@ -1166,7 +1174,7 @@ int hb_ens_init(hb_ens *e, double tsys, double eta, double eta_s, double dtmax)
         std::memset(&t, 0, sizeof t);
         t.tsys = tsys;
     }
-    ce = cudaMemcpy(e->d_cstate, cs.data(), cs.size() * sizeof(TeamState), cudaMemcpyHostToDevice);
+    ce = upload(e, e->d_cstate, cs.data(), cs.size() * sizeof(TeamState));
     if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "cluster state", ce);
     e->groups_ready = false;
     e->ready = true;
@@ -1195,7 +1203,7 @@ int hb_ens_run(hb_ens *e, double tend, long long max_block_steps)
     if (s0 != HB_OK) return s0;
     volatile EnsStatus *st = e->h_st;
     if (!(tend >= st->tsys)) return ens_fail(e, HB_ERR_INVALID, "tend is before tsys");
-    ce = cudaMemcpy(&e->d_s->tend, &tend, sizeof(double), cudaMemcpyHostToDevice);
+    ce = upload(e, &e->d_s->tend, &tend, sizeof(double));
     if (ce != cudaSuccess) return ens_fail(e, HB_ERR_CUDA, "tend upload", ce);
     {
         const int nb = std::max(1, std::min((e->nslot + 255) / 256, e->nsm * 8));
@@ -1278,8 +1286,7 @@ int hb_ens_cluster_engine(hb_ens *e, int c, int *engine, int *team_ctas)
 int hb_ens_energy(hb_ens *e, double *kinetic, double *potential)
 {
     if (!e || !kinetic || !potential) return HB_ERR_INVALID;
-    cudaError_t ce = cudaMemcpy(e->d_cl, e->cl.data(), e->cl.size() * sizeof(Cluster),
-                                cudaMemcpyHostToDevice);
+    cudaError_t ce = upload(e, e->d_cl, e->cl.data(), e->cl.size() * sizeof(Cluster));
     if (ce == cudaSuccess) {
         switch (e->order) {
         case 4: ce = ens_energy<4>(e->L, e->d_pot, e->d_eout, e->stream); break;
