@@ -319,11 +319,10 @@ constexpr size_t kZeroCopyBytes = 256 << 10;
 // since contexts that never move most of a large system have no use for it.  Smaller
 // calls use the slices' buffer, before and after it is made alike: the scratch sets
 // the bands, hence the association of the sums, and a call's bits may not depend on
-// the calls before it.  Large calls use that buffer too, all of them, when the memory
-// is full, and those in a capture before the first other one, which may not allocate.
-// 6th order, all active, that buffer against this scratch: N = 20000 1.12 / 1.08
-// ms, 32768 2.88 / 2.66, 65536 12.4 / 10.9, 131072 (32 rows up to 256 MiB) 40.0 /
-// 39.3.  Making it took 0 to 4 ms.
+// the calls before it.  When the memory is full, large calls use that buffer too,
+// all of them.  6th order, all active, that buffer against this scratch: N = 20000
+// 1.12 / 1.08 ms, 32768 2.88 / 2.66, 65536 12.4 / 10.9, 131072 (32 rows up to 256 MiB)
+// 40.0 / 39.3.  Making it took 0 to 4 ms.
 constexpr long long kRowsPairs = 1LL << 30;
 
 struct Scratch {
@@ -335,16 +334,19 @@ Scratch pairs_once_scratch(hb_ctx *c, int nact)
 {
     const Scratch small{c->d_partial, c->partial_cap};
     if ((long long)nact * c->npad < kRowsPairs) return small;
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (!c->rows_tried && cudaStreamIsCapturing(c->stream, &st) == cudaSuccess &&
-        st == cudaStreamCaptureStatusNone) {
+    if (!c->rows_tried) {
         c->rows_tried = true;
         const size_t want = std::min((size_t)64 * c->npad * c->F, (size_t)64 << 20);
         if (want > c->partial_cap) {
+            // An allocation is no part of any stream: in the relaxed mode it neither
+            // fails under nor breaks a capture, this stream's or another thread's.
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            const bool relaxed = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
             if (cudaMalloc((void **)&c->d_rows, want * sizeof(double)) == cudaSuccess)
                 c->rows_cap = want;
             else
                 (void)cudaGetLastError();
+            if (relaxed) cudaThreadExchangeStreamCaptureMode(&mode);
         }
     }
     return c->rows_cap ? Scratch{c->d_rows, c->rows_cap} : small;

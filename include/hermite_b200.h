@@ -95,7 +95,11 @@ int hb_predict_all(hb_ctx *ctx, double tsys);
  * SRC/hermite4-titan.cu:362-412, SRC/hermite6-titan.cu:362-405,
  * SRC/hermite8-titan.cu:428-473.  Force on slots [0,nact) from all slots,
  * self pair included (exactly zero for eps2 > 0).  Writes nact force records
- * to force_out and returns when they are there.  0 <= nact <= nbody. */
+ * to force_out and returns when they are there.  0 <= nact <= nbody.
+ * A context's first 4th- or 6th-order FP64 call of at least 2^30 pairs (nact times
+ * the padded slots), this one or hb_force_device, allocates up to 512 MiB of
+ * device memory, kept until hb_destroy; it may do so while a stream is being
+ * captured.  Without that memory such calls still run, in more passes. */
 int hb_force_first_nact(hb_ctx *ctx, int nact, double eps2, double *force_out);
 
 /* Gravity::calc_potential(double eps2, double potbuf[]) --
