@@ -136,7 +136,7 @@ def load_library() -> ctypes.CDLL:
         raise RuntimeError(f"{path} is missing: build it with `python -m hermite_b200.build`")
     lib = ctypes.CDLL(str(path))
     P, I, D = ctypes.c_void_p, ctypes.c_int, ctypes.c_double
-    dp = P          # double *: takes an address or any ctypes pointer to doubles
+    dp = ctypes.POINTER(ctypes.c_double)
     sig = {
         "hb_create": (I, [I, I, I, ctypes.POINTER(P)]),
         "hb_destroy": (I, [P]),
@@ -212,13 +212,13 @@ def load_library() -> ctypes.CDLL:
 
 
 def _dptr(a: np.ndarray):
-    """An array's data as a pointer argument.  By the buffer protocol, a fifth
+    """An array's data as a `double *` argument.  By the buffer protocol, a fifth
     of the 1.5 us of ndarray.ctypes.data_as, which a block step pays twice;
-    read-only and empty arrays, which that refuses, by address."""
+    read-only and empty arrays, which that refuses, the long way."""
     try:
-        return ctypes.byref(ctypes.c_char.from_buffer(a))
+        return ctypes.byref(ctypes.c_double.from_buffer(a))
     except (TypeError, ValueError):
-        return a.ctypes.data
+        return a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
 
 
 def _out_buffer(out, rows: int, cols: int | None = None) -> np.ndarray:
