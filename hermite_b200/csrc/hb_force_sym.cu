@@ -42,7 +42,8 @@ int bands_t(int ca, int nchunk, size_t cap, int nsm)
     int bands = 0;
     for (int g0 = 0; g0 * SymShape<ORDER>::GC < ca; ++bands) {
         const Band b = band_from<ORDER>(g0, ca, nchunk, room, nsm);
-        if (b.ng < 1) return -1;
+        // its rows and slice sums have to fit
+        if (b.ng < 1 || b.ng * (ca + (long long)b.smax * SymShape<ORDER>::GC) > room) return -1;
         g0 += b.ng;
     }
     return bands;
