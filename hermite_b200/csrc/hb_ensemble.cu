@@ -686,14 +686,28 @@ cudaError_t upload(hb_ens *e, void *dst, const void *src, size_t bytes)
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, e->stream);
 }
 
-// Team size for a cluster of n particles: a CTA per kEnsTeamSlots, more if its
-// slots do not fit the CTAs' shared memory; a function of n alone, so that a
-// cluster's sums do not depend on the other clusters.  Smaller teams use the
-// GPU better where there are many clusters, larger ones end sooner where there
-// are few (ms, 32 clusters of 256 ... 4096 particles at 4th order / 256 of them at
-// 6th order): 512 slots per CTA 18.6 / 45.8, 448 16.8 / 44.0, 384 15.5 / 49.1, 320
-// 13.5 / 55.9; powers of two from 512 on, one group after another, 43.0 / 50.7.
-constexpr int kEnsTeamSlots = 384;
+// Team size for a cluster of n particles, more if its slots do not fit the CTAs'
+// shared memory; a function of n and the engine asked for, so that a cluster's sums
+// do not depend on the other clusters.
+//
+// The automatic engine takes powers of two, of 512 slots per CTA at most.  Where
+// there are many clusters of one size, their number at work at once decides, and a
+// cluster of thread blocks has to fit one processing cluster of the GPU, which
+// odd sizes leave part empty.  A CTA per 384 slots, against it (ms, 4th order, equal
+// clusters): 74 of 4096 213 / 119, 148 of 1024 16.2 / 12.0, 296 of 400 6.1 / 4.6,
+// 37 of 4096 at 6th order 45.2 / 28.0.  Few clusters of many sizes end sooner with
+// it (32 of 256 ... 4096 15.5 / 18.7, one of 512 1.35 / 2.17); the team engine asked
+// for by name, which does not weigh engines against one another, takes it.
+constexpr int kEnsTeamSlots = 384, kEnsAutoSlots = 512;
+
+int ens_team_size(int engine, int n)
+{
+    if (engine == HB_ENGINE_TEAM) return std::min(16, (n + kEnsTeamSlots - 1) / kEnsTeamSlots);
+    int C = 1;
+    while (C < 16 && (long long)C * kEnsAutoSlots < n) C <<= 1;
+    return C;
+}
+
 constexpr long long kEnsTeamStepsPerLaunch = 1LL << 14;
 
 int build_groups(hb_ens *e)
@@ -727,9 +741,7 @@ int build_groups(hb_ens *e)
     for (int c = 0; c < e->nclusters; ++c) {
         const int n = e->cl[c].n, nch = (n + 31) / 32;
         int C = e->team_ctas;
-        if (C == 0) {
-            C = std::min(16, (n + kEnsTeamSlots - 1) / kEnsTeamSlots);
-        }
+        if (C == 0) C = ens_team_size(e->engine, n);
         for (;;) {
             const TeamConfig *cf = cfg_for(C);
             // the automatic choice takes only clusters whose records fit in
