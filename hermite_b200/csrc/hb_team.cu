@@ -541,8 +541,15 @@ int team_shape_t(const TeamConfig &cfg, int nmax, TeamLaunch *L)
                    (long long)SM::per_i;
     // every slot of the team where that fits, so that no step overflows the
     // push regions: at N = 1024, 4th order, 6 % of the steps did with 512 and took
-    // 33 us each in the pull path, 2 us of the mean step
-    im = std::min<long long>(im & ~31LL, std::max((long long)kTeamWarps * 32, (long long)jl * cfg.ctas));
+    // 33 us each in the pull path, 2 us of the mean step.  Else whole passes of the
+    // CTA's threads (of two i each at 4th order): a round of 1184 takes three
+    // half-empty passes' time where 1024 takes one (eight CTAs, N = 4096, 4th order)
+    constexpr int kPass = kTeamWarps * 32;
+    const long long all = std::max((long long)kPass, (long long)jl * cfg.ctas);
+    im &= ~31LL;
+    if (im >= all) im = all;
+    else if (ORDER == 4 && im >= 2 * kPass) im -= im % (2 * kPass);
+    else if (im >= kPass) im -= im % kPass;
     if (im < (rsmem ? kTeamIMax : kTeamIMinGlobal)) return -1;
     L->ctas = cfg.ctas;
     L->jl_cap = jl;
