@@ -369,16 +369,22 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
                     });
                 team.sync();   // barrier 3: every partial is with its owner
 
-                if (w == 0) {
-                    // the ranks' partials in rank order, one value per lane
-                    for (int e = lane; e < kact * F; e += 32) {
+                // the ranks' partials in rank order, one value per thread, then the
+                // corrector: by warp 0 (no CTA barrier) up to one own active slot
+                // per lane, by all threads above (a run of N = 1024 on two CTAs, 4th
+                // order: 4.96 ms by warp 0 alone, 4.77 this way)
+                const int nt = kact > 32 ? T : 32;
+                if (tid < nt)
+                    for (int e = tid; e < kact * F; e += nt) {
                         double v = part[e];
 #pragma unroll 4
                         for (int src = 1; src < C; ++src) v += part[(size_t)src * KM * F + e];
                         part[e] = v;
                     }
-                    __syncwarp();
-                    for (int a = lane; a < kact; a += 32) {
+                if (nt == T) __syncthreads();
+                else __syncwarp();
+                if (tid < nt)
+                    for (int a = tid; a < kact; a += nt) {
                         double f[F];
 #pragma unroll
                         for (int k = 0; k < F; ++k) f[k] = part[a * F + k];
@@ -391,9 +397,9 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
                         dts[q] = dtn;
                         tn[q] = dtn + r[7];
                     }
-                    __syncwarp();
-                    find_candidates();
-                }
+                if (nt == T) __syncthreads();
+                else __syncwarp();
+                if (w == 0) find_candidates();
                 __syncthreads();
                 announce();
             } else {
