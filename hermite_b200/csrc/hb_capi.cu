@@ -1071,15 +1071,17 @@ int hb_integrator_restore(hb_ctx *ctx, const char *path, double eps2, double eta
 namespace {
 constexpr long long kTeamStepsPerLaunch = 1LL << 14;
 
-// The team size for one system of n slots: a CTA per 32-slot chunk, at most
-// 16 CTAs (8 where the device cannot co-schedule a 16-CTA cluster with this
-// kernel's shared memory).  Two chunks per CTA measured slower: N = 200 4.7
-// against 4.3 us per block step, N = 512 5.4 against 5.3.
+// The team size for one system of n slots: the smallest that gives no CTA more
+// 32-slot chunks than 16 CTAs would (8 where the device cannot co-schedule a
+// 16-CTA cluster with this kernel's shared memory), a CTA per chunk up to 16.  More
+// CTAs only add to the barriers and pushes: N = 700 on 11 / 16 CTAs 5.9 / 6.3 us per
+// block step at 4th order, 13.8 / 16.8 at 8th; N = 1100 on 12 / 16 6.9 / 7.1 and 29.1 /
+// 30.2.  Two chunks per CTA below 16 measured slower: N = 150 5.3 against 4.6 us.
 int team_config_for(hb_ctx *ctx, int n, int want_ctas, TeamConfig *cfg)
 {
     const int nch = (n + 31) / 32;
-    int ctas = want_ctas > 0 ? want_ctas
-                             : std::min(16, nch);
+    const int per = (nch + 15) / 16;       // chunks per CTA
+    int ctas = want_ctas > 0 ? want_ctas : (nch + per - 1) / per;
     for (;;) {
         const cudaError_t e = team_setup(ctx->order, ctas, cfg);
         if (e == cudaSuccess && cfg->max_teams >= 1) break;

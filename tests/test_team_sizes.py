@@ -1,11 +1,11 @@
-"""The automatic ensemble engine's team sizes: powers of two of at most 512 slots
+"""Team sizes chosen by the library.  Ensembles: powers of two of at most 512 slots
 per CTA, which fill the GPU where many clusters are of one size (a CTA per 384
 slots took up to 1.8 times as long there), and the same results as teams of that
 size asked for."""
 import numpy as np
 import pytest
 
-from hermite_b200 import Ensemble
+from hermite_b200 import Ensemble, Gravity
 from hermite_b200.ic import plummer, records
 
 pytestmark = pytest.mark.gpu
@@ -29,3 +29,10 @@ def test_same_as_asked_for():
             e.run(1 / 128)
             out.append([e.get_cluster(c) for c in range(2)])
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("n,ctas", [(1, 1), (33, 2), (512, 16), (513, 9), (700, 11), (1024, 16), (1025, 11), (2560, 16)])
+def test_single_system(n, ctas):
+    """No more CTAs than the chunks per CTA of the largest team call for."""
+    with Gravity(8, n) as g:
+        assert g.engine() == ("team", ctas)
