@@ -219,7 +219,7 @@ potential_kernel(const double *__restrict__ posm, int nchunk, int n, double eps2
     constexpr int TB = kPotTileChunks * kPosmChunkBytes;
     __shared__ __align__(128) unsigned char ring[2 * TB];
     __shared__ __align__(8) uint64_t bar[2];
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
     const int i = blockIdx.x * kPotThreads + tid;   // < npad always
     const double *ci = posm + (size_t)(i >> 5) * NC * 32 + (i & 31);
     const double xi = ci[0], yi = ci[32], zi = ci[64];
@@ -266,21 +266,32 @@ potential_kernel(const double *__restrict__ posm, int nchunk, int n, double eps2
         const double *tile = reinterpret_cast<const double *>(ring + (t & 1) * TB);
         for (int q = 0; q < cnt; ++q) {
             const double *cp = tile + q * NC * 32;
-            const int jbase = (c0 + t * kPotTileChunks + q) * 32;
-            double part = 0.0;
+            // The self pair is left out, by index, in the one chunk that holds it.
+            // (Looking for it in every chunk, by a branch around the rsqrt, took
+            // 48 us instead of 34 at N = 100, and 24.1 ms instead of 20.4 at N =
+            // 131072 in double-double.)
+            auto pairs = [&](auto diag) {
+                double part = 0.0;
 #pragma unroll 8
-            for (int jl = 0; jl < 32; ++jl) {
-                double dx = cp[jl] - xi, dy = cp[32 + jl] - yi, dz = cp[64 + jl] - zi;
-                if constexpr (NC == 7) {
-                    dx = dx + (cp[128 + jl] - xli);
-                    dy = dy + (cp[160 + jl] - yli);
-                    dz = dz + (cp[192 + jl] - zli);
+                for (int jl = 0; jl < 32; ++jl) {
+                    double dx = cp[jl] - xi, dy = cp[32 + jl] - yi, dz = cp[64 + jl] - zi;
+                    if constexpr (NC == 7) {
+                        dx = dx + (cp[128 + jl] - xli);
+                        dy = dy + (cp[160 + jl] - yli);
+                        dz = dz + (cp[192 + jl] - zli);
+                    }
+                    double r2 = fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2)));
+                    double mj = cp[96 + jl];
+                    if (diag.value && jl == lane) {      // any finite rsqrt, no mass
+                        r2 = 1.0;
+                        mj = 0.0;
+                    }
+                    part = fma(-mj, rsqrt_fp64(r2), part);
                 }
-                const double r2 = fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2)));
-                const double ri = (jbase + jl == i) ? 0.0 : rsqrt_fp64(r2);
-                part = fma(-cp[96 + jl], ri, part);
-            }
-            total += part;
+                total += part;
+            };
+            if (c0 + t * kPotTileChunks + q == (i >> 5)) pairs(std::true_type());
+            else pairs(std::false_type());
         }
         __syncthreads();
         if (tid == 0 && t + 2 < ntile) issue(t + 2);
