@@ -241,23 +241,37 @@ const TuneEntry *lookup_tuning(int order, bool mixed, int n, int nact)
 // the last CTA of an i-tile could add alone, hence launch_reduce.
 //
 // Shape 11 halves the padding of nact to whole i-tiles and the chunks a warp
-// takes in turn; it wins up to 64 particles and where all pairs together are
-// few (N = 32768, 6th order, nact = 300: 48.6 against 51.3 us; N = 262144,
-// nact = 500: 493 against 480 us).
+// takes in turn; it wins where all pairs together are few (N = 32768, 6th order,
+// nact = 300: 48.6 against 51.3 us; N = 262144, nact = 500: 493 against 480 us).
 //
 // Up to 3072 slots the launches themselves matter: shape 13 (four warps, 32
 // particles) predicts what it streams and saves the predictor's launch (block
 // steps of N = 600, 8th order, nact = 17: 31.7 against 36.9 us; N = 1346, nact = 336 35.6
-// against 40.0; N = 4000, all active 229 against 221).
-constexpr int kShapeWide = 8, kShapeNarrow = 11, kShapeFused = 13;
+// against 40.0; N = 4000, all active 229 against 221).  Up to 160 particles of any
+// number of slots the predictor's pass over memory does: shape 13 in one wave, or two
+// for several tiles, against the two-pass shapes (8th order, N = 262144, nact = 17 / 64 /
+// 160: 78 / 129 / 292 us against 100 / 156 / 336; 4th order mixed, N = 2^20, nact = 1:
+// 81 against 115; equal to 2 % at N = 131072, nact = 129 ... 160, slower beyond).
+//
+// Double-double positions take more registers: four warps, 64 particles sharing
+// tiles by pairs of warps (shape 3), or 128 (shape 0) where that pads nact no
+// further, are 2-6 % faster there than shapes 11 and 8 (N = 8192, nact = 1024 100
+// against 105 us; N = 32768, all active 7.04 against 7.46 ms).  At 8th order shape
+// 3 takes small steps of up to 8192 slots (N = 4096, nact = 500 50 against 54 us, N = 8192,
+// nact = 3000 235 against 251; N = 16384, nact = 400 83 against 80).
+constexpr int kShapeWide = 8, kShapeNarrow = 11, kShapeFused = 13, kShapePairs = 3, kShapeWideDD = 0;
 constexpr long long kNarrowUnits = 12288;      // 64-particle tiles x chunks
-constexpr int kFusedSlots = 3072;
+constexpr int kFusedSlots = 3072, kFusedAct = 160, kPairsSlots = 8192;
 
 int auto_variant(const hb_ctx *c, int nact)
 {
-    if (c->npad <= kFusedSlots) return kShapeFused;
-    const long long units = (long long)((nact + 63) / 64) * (c->npad / 32);
-    return nact <= 64 || units <= kNarrowUnits ? kShapeNarrow : kShapeWide;
+    const bool mixed = c->pred_precision == HB_MIXED;
+    if (c->npad <= kFusedSlots || nact <= kFusedAct) return kShapeFused;
+    const int tiles = (nact + 63) / 64;
+    const bool narrow = (long long)tiles * (c->npad / 32) <= kNarrowUnits;
+    if (c->order == 9) return !narrow && (tiles % 2 == 0 || nact >= 2048) ? kShapeWideDD : kShapePairs;
+    if (c->order == 8 && !mixed && narrow && c->npad <= kPairsSlots) return kShapePairs;
+    return narrow ? kShapeNarrow : kShapeWide;
 }
 
 // j-slices of the automatic shape; `resident` CTAs of it run at once.
@@ -272,7 +286,9 @@ int auto_slices(int v, int gx, int nchunk, int resident)
     // (8th order, N = 2500, nact = 625: 49.4 us; slices of 3 and 4 chunks in turn 61.3).
     double c;
     if (v == kShapeFused)
-        c = 4;           // one per warp
+        c = std::max(4.0, gx == 1 ? x : std::min(x, std::max(8.0, x / 2)));
+    else if (v == kShapePairs)
+        c = 4;
     else if (v == kShapeNarrow)
         c = 2 * std::max(1, std::min(4, std::max((int)(0.6 * std::sqrt(x) + 0.5), nchunk / 512)));
     else
