@@ -200,7 +200,8 @@ int sync_stream(hb_ctx *ctx)
 }
 
 // Launch shapes measured by hermite_b200/autotune.py on a B200, keyed by
-// (order, precision, log2 N bucket, log2 nact bucket).
+// (order, precision, log2 N bucket, log2 nact bucket); only a caller that fixes the
+// slice count and not the shape gets them.
 struct TuneEntry {
     int order, mixed, log2n, log2nact, variant, jsplit;
 };
@@ -297,27 +298,15 @@ int auto_slices(int v, int gx, int nchunk, int resident)
     return std::max(1, (int)(nchunk / c));
 }
 
-// Launch shape for a given slice count (hb_set_force_shape with an automatic
-// shape): the tuned variant and j-slice count of
-// the nearest bucket (the slice count rescaled to keep the measured number
-// of CTAs), else a heuristic; then the slice count is clamped so that each
-// CTA keeps at least 8 chunks and the partials fit in the scratch buffer.
-int pick_variant(const hb_ctx *c, int nact, int *jsplit_hint)
+// The shape when the caller fixes the slice count alone (hb_set_force_shape with an
+// automatic shape): that of the nearest measured bucket, else by nact.
+int pick_variant(const hb_ctx *c, int nact)
 {
-    *jsplit_hint = 0;
     if (c->variant_override >= 0) return c->variant_override;
     const bool mixed = c->pred_precision == HB_MIXED;
     // double-double (order 9) uses the 8th-order measurements
-    if (const TuneEntry *e = lookup_tuning(c->order == 9 ? 8 : c->order, mixed, c->nbody, nact)) {
-        const ForceVariant *fv = force_variant(c->order, mixed, e->variant);
-        if (fv) {
-            const long long gx_bucket = ((1LL << e->log2nact) + fv->ti - 1) / fv->ti;
-            const long long gx = (nact + fv->ti - 1) / fv->ti;
-            const long long ctas = gx_bucket * e->jsplit;
-            *jsplit_hint = (int)std::max<long long>(1, (ctas + gx - 1) / gx);
-            return e->variant;
-        }
-    }
+    if (const TuneEntry *e = lookup_tuning(c->order == 9 ? 8 : c->order, mixed, c->nbody, nact))
+        if (force_variant(c->order, mixed, e->variant)) return e->variant;
     if (nact <= 32) return 2;
     if (nact <= 64) return 3;
     if (nact <= c->nsm * 256) return 0;
@@ -416,8 +405,7 @@ int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
         ctx->launches += launches;
         return HB_OK;
     }
-    int jsplit_hint = 0;
-    const int v = automatic ? auto_variant(ctx, nact) : pick_variant(ctx, nact, &jsplit_hint);
+    const int v = automatic ? auto_variant(ctx, nact) : pick_variant(ctx, nact);
     const ForceVariant *fv = force_variant(ctx->order, mixed, v);
     if (!fv) return fail(ctx, HB_ERR_INVALID, "force variant %d does not exist", v);
     const int m = mixed ? 1 : 0;
@@ -434,15 +422,13 @@ int run_force(hb_ctx *ctx, int nact, double eps2, double *force_out_dev)
     int S;
     if (automatic) {
         S = auto_slices(v, gx, nchunk, ctx->nsm * ctx->blocks_per_sm[m][v]);
+    } else if (ctx->jsplit_override > 0) {
+        S = std::min(ctx->jsplit_override, nchunk);
     } else {
-        S = ctx->jsplit_override > 0 ? ctx->jsplit_override : jsplit_hint;
-        if (S <= 0) {
-            const int target = ctx->nsm * ctx->blocks_per_sm[m][v];
-            S = gx >= target ? 1 : (target + gx - 1) / gx;
-            // at least 8 chunks (256 j) per CTA and 2 chunks per j-warp
-            S = std::min(S, std::max(1, nchunk / std::max(8, 2 * fv->wj)));
-        }
-        S = std::max(1, std::min(S, ctx->jsplit_override > 0 ? nchunk : std::max(1, nchunk / 8)));
+        // one wave, at least 8 chunks (256 j) per CTA and 2 chunks per j-warp
+        const int target = ctx->nsm * ctx->blocks_per_sm[m][v];
+        S = gx >= target ? 1 : (target + gx - 1) / gx;
+        S = std::min(S, std::max(1, nchunk / std::max(8, 2 * fv->wj)));
     }
     if (S > 1) {
         const size_t need_per_slice = (size_t)gx * fv->ti * ctx->F;

@@ -2,7 +2,7 @@
 //
 // Replaces force_kernel + reduce_kernel of the reference's CUDA path
 // (SRC/hermite4-titan.cu:189-238,303-327; SRC/hermite6-titan.cu:245-299,
-// 302-326; SRC/hermite8-titan.cu:304-364,367-391) with one kernel:
+// 302-326; SRC/hermite8-titan.cu:304-364,367-391):
 //
 //   grid  = (i-tiles, j-slices S); block = NW warps.
 //   * j-particles stream through shared memory in tiles of TCH 32-slot
@@ -12,10 +12,11 @@
 //     the CTA's NW warps form WI = NW/WJ i-groups, and the WJ warps of an
 //     i-group split each j tile between them (small-nact occupancy).
 //   * j-slices of one i-tile are separate CTAs (blockIdx.y), as the
-//     reference's NJBLOCK; their FP64 partials meet in a scratch buffer and
-//     the last CTA of the i-tile to finish adds them in slice order -- no
-//     second launch, and the sum order is fixed, so results are
-//     deterministic for a given launch shape.
+//     reference's NJBLOCK; their FP64 partials meet in a scratch buffer.  A
+//     chained launch adds them (launch_reduce; the automatic shape, which
+//     cuts many slices), or the last CTA of the i-tile to finish does, in
+//     slice order (explicit shapes and the no-allocation entry).  Either
+//     order is fixed, so results are deterministic for a given launch shape.
 #pragma once
 #include <type_traits>
 #include "hb_common.cuh"

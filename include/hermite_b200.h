@@ -160,13 +160,15 @@ long long hb_launch_count(const hb_ctx *ctx);
 int hb_set_wait_limit(hb_ctx *ctx, long long polls);
 
 /* Launch shape of the force kernel, picked per (order, precision, nbody,
- * nact) by the built-in tuning table unless overridden here.  variant
- * indexes the compiled kernel variants (see hb_force_variant_count);
- * jsplit is the number of j-slices (CTAs per i-tile); 0 means "auto".
- * With variant < 0 (automatic), FP64 block steps of at most 16 active
- * particles (orders 4, 6, 8) take a separate kernel in which the lanes of
- * a warp share an i-particle and split the j range; an explicit variant
- * always takes the tiled kernel. */
+ * nact) by a rule on the sizes unless overridden here.  variant indexes the
+ * compiled kernel variants (see hb_force_variant_count); jsplit is the number
+ * of j-slices (CTAs per i-tile); 0 means "auto".  With variant < 0
+ * (automatic), FP64 block steps of at most 16 active particles (orders 4, 6,
+ * 8) take a separate kernel in which the lanes of a warp share an i-particle
+ * and split the j range; with jsplit 0 too, 4th- and 6th-order FP64 steps in
+ * which most particles are active take each pair once.  An explicit variant
+ * always takes the tiled kernel; jsplit alone takes it in a measured table's
+ * variant. */
 int hb_set_force_shape(hb_ctx *ctx, int variant, int jsplit);
 int hb_force_variant_count(int order, int precision);
 /* Describe a variant: threads per CTA, i per thread, warps splitting j. */
@@ -204,7 +206,7 @@ int hb_integrator_init(hb_ctx *ctx, double tsys, double eps2, double eta, double
  *                   launch; the same block steps and records as the graph
  *                   engine, bit for bit (any N, FP64 or mixed);
  *  HB_ENGINE_TEAM   one thread-block cluster of up to 16 CTAs runs the whole
- *                   block-step loop in one kernel, three cluster barriers per
+ *                   block-step loop in one kernel, two cluster barriers per
  *                   step (FP64; N up to 16 x the slots one CTA holds in
  *                   shared memory, about 16k);
  *  HB_ENGINE_AUTO   the team engine for FP64 systems of up to 2560
