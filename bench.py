@@ -251,7 +251,7 @@ def run_reference(args):
 
 # ---------------------------------------------------------------------------
 def traffic_from_profiles(name):
-    """dram bytes per force-kernel launch from a committed ncu summary."""
+    """dram bytes of one force call from a committed ncu summary."""
     p = ROOT / "profiles" / name
     if not p.exists():
         return None
