@@ -160,6 +160,17 @@ __device__ __forceinline__ void team_force(const double *ibuf, const double *pre
     team_force_ni<ORDER, 1>(ibuf, pred, JL, nr, ng, eps2, idx, out);
 }
 
+// A round of the pull path for im i-states: whole passes of the CTA's threads, of two
+// i each at 4th order.  A round of 1184 takes two passes where 1024 takes one (eight
+// CTAs, N = 4096, 4th order: 129 against 118 ms for 74 clusters).
+template <int ORDER>
+__host__ __device__ __forceinline__ int team_pass(int im)
+{
+    constexpr int kPass = kTeamWarps * 32;
+    if (ORDER == 4 && im >= 2 * kPass) return im / (2 * kPass) * (2 * kPass);
+    return im >= kPass ? im / kPass * kPass : im;
+}
+
 template <int ORDER, bool RSMEM>
 __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
 {
@@ -403,16 +414,19 @@ __global__ void __launch_bounds__(kTeamWarps * 32, 1) team_kernel(TeamLaunch L)
                 __syncthreads();
                 announce();
             } else {
-                // many actives: rounds pulled from the owners.  The lanes per
-                // i-particle are chosen from the rounds of misc[2] that the system has
-                // when it is alone in a launch; IM, which comes from the largest
-                // system of this one, only cuts those in parts.  So a system's sums,
-                // here and above, do not depend on the others (IM is above misc[2]
-                // only where that holds every slot).
+                // many actives: rounds pulled from the owners, of whole passes (team_pass).
+                // The lanes per i-particle are chosen as where the system is alone in a
+                // launch: one choice up to misc[2] active states, which is what IM is
+                // there, by its rounds above.  IM itself comes from the largest system
+                // of this launch and only cuts those in parts.  So a system's sums, here
+                // and above, do not depend on the others (IM is above misc[2] only where
+                // that holds every slot).
                 team.sync();   // barrier 2: predicted states and candidate lists complete
-                for (int r0 = 0; r0 < nact; r0 += misc[2])
-                for (int base = r0; base < min(r0 + misc[2], nact); base += IM) {
-                    const int nr = min(IM, min(r0 + misc[2], nact) - base), ng = min(misc[2], nact - r0);
+                const int step = nact <= misc[2] ? nact : team_pass<ORDER>(misc[2]);
+                for (int r0 = 0; r0 < nact; r0 += step)
+                for (int base = r0; base < min(r0 + step, nact); base += team_pass<ORDER>(IM)) {
+                    const int nr = min(team_pass<ORDER>(IM), min(r0 + step, nact) - base);
+                    const int ng = min(step, nact - r0);
                     for (int i = tid; i < nr; i += T) {
                         const int g = base + i;
                         int c = 0;
@@ -547,15 +561,14 @@ int team_shape_t(const TeamConfig &cfg, int nmax, TeamLaunch *L)
                    (long long)SM::per_i;
     // every slot of the team where that fits, so that no step overflows the
     // push regions: at N = 1024, 4th order, 6 % of the steps did with 512 and took
-    // 33 us each in the pull path, 2 us of the mean step.  Else whole passes of the
-    // CTA's threads (of two i each at 4th order): a round of 1184 takes three
-    // half-empty passes' time where 1024 takes one (eight CTAs, N = 4096, 4th order)
-    constexpr int kPass = kTeamWarps * 32;
-    const long long all = std::max((long long)kPass, (long long)jl * cfg.ctas);
-    im &= ~31LL;
-    if (im >= all) im = all;
-    else if (ORDER == 4 && im >= 2 * kPass) im -= im % (2 * kPass);
-    else if (im >= kPass) im -= im % kPass;
+    // 33 us each in the pull path, 2 us of the mean step
+    const long long all = std::max((long long)kTeamWarps * 32, (long long)jl * cfg.ctas);
+    im = std::min<long long>(im & ~31LL, all);
+    // and whole passes where little of another is left: a pushed step of that size
+    // takes the pass for it (4th order, 74 clusters of 4096 122 against 118 ms; double-
+    // double, N = 2560 43.8 against 42.6 us per block step)
+    const int whole = team_pass<ORDER>((int)im);
+    if (im < all && im - whole <= kTeamWarps * 16) im = whole;
     if (im < (rsmem ? kTeamIMax : kTeamIMinGlobal)) return -1;
     L->ctas = cfg.ctas;
     L->jl_cap = jl;
