@@ -4,7 +4,8 @@ For each (order, precision, N bucket, nact bucket) it times every compiled
 kernel variant (threads per CTA, i-chunks per warp, in-CTA j split, tile
 depth, register cap) and several j-slice counts S, on the current GPU, and
 writes the fastest choice to hermite_b200/csrc/hb_tuning.inc, which the
-library compiles in (hb_capi.cu looks up the nearest bucket).
+library compiles in.  hb_capi.cu takes the nearest bucket's variant where a caller
+fixes the slice count alone; the automatic shape is a rule on the sizes.
 
     python -m hermite_b200.autotune [--out hermite_b200/csrc/hb_tuning.inc]
                                     [--json results.json] [--quick]

@@ -40,7 +40,9 @@ constexpr int kMaxBody = 1 << 24;
 // hb_set_jp_records of at least this many bytes uploads at once, in chunks.
 constexpr size_t kEagerUploadBytes = (size_t)4 << 20, kUploadChunkBytes = (size_t)2 << 20;
 // HB_ENGINE_AUTO takes the team engine up to this many particles (4th order, us
-// per block step, team against graph: N = 2048 9.7 / 11.9, 2500 11.7 / 12.3, 3000 17.7 / 13.8).
+// per block step, team against graph: N = 2048 8.4 / 11.4, 2560 10.8 / 12.0, 2950 15.7 /
+// 13.0).  The graph engine is the faster from about 1500 on at 6th order (N = 2048 16.7 /
+// 13.7) and 1024 at 8th (28.8 / 17.8).
 constexpr int kTeamAutoMaxBody = 2560;
 
 int rec_words(int order) { return 8 + 3 * (order - 2); }

@@ -694,10 +694,10 @@ cudaError_t upload(hb_ens *e, void *dst, const void *src, size_t bytes)
 // there are many clusters of one size, their number at work at once decides, and a
 // cluster of thread blocks has to fit one processing cluster of the GPU, which
 // odd sizes leave part empty.  A CTA per 384 slots, against it (ms, 4th order, equal
-// clusters): 74 of 4096 213 / 119, 148 of 1024 16.2 / 12.0, 296 of 400 6.1 / 4.6,
-// 37 of 4096 at 6th order 45.2 / 28.0.  Few clusters of many sizes end sooner with
-// it (32 of 256 ... 4096 15.5 / 18.7, one of 512 1.35 / 2.17); the team engine asked
-// for by name, which does not weigh engines against one another, takes it.
+// clusters): 74 of 4096 206 / 119, 148 of 1024 15.8 / 12.0, 296 of 400 5.9 / 4.5,
+// 37 of 4096 at 6th order 43.5 / 27.4.  Few clusters end sooner with it (32 of 256 ...
+// 4096 22.3 / 26.1, one of 512 1.30 / 2.11); the team engine asked for by name, which
+// does not weigh engines against one another, takes it.
 constexpr int kEnsTeamSlots = 384, kEnsAutoSlots = 512;
 
 int ens_team_size(int engine, int n)
