@@ -49,7 +49,7 @@ def test_first_large_call_captured(plain):
         g.set_stream(s.cuda_stream)
         g.set_jp_records(rec)
         g.predict_all(0.0)
-        g.force_device(100, EPS2)           # the predictor pass, not of the graph
+        g.predict_pass()                    # not of the graph
         g.synchronize()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph, stream=s):
