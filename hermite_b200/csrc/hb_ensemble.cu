@@ -690,14 +690,16 @@ cudaError_t upload(hb_ens *e, void *dst, const void *src, size_t bytes)
 // shared memory; a function of n and the engine asked for, so that a cluster's sums
 // do not depend on the other clusters.
 //
-// The automatic engine takes powers of two, of 512 slots per CTA at most.  Where
-// there are many clusters of one size, their number at work at once decides, and a
-// cluster of thread blocks has to fit one processing cluster of the GPU, which
-// odd sizes leave part empty.  A CTA per 384 slots, against it (ms, 4th order, equal
-// clusters): 74 of 4096 206 / 119, 148 of 1024 15.8 / 12.0, 296 of 400 5.9 / 4.5,
-// 37 of 4096 at 6th order 43.5 / 27.4.  Few clusters end sooner with it (32 of 256 ...
-// 4096 22.3 / 26.1, one of 512 1.30 / 2.11); the team engine asked for by name, which
-// does not weigh engines against one another, takes it.
+// The automatic engine takes powers of two, of 512 slots per CTA at most, and nine
+// CTAs in place of eight.  Where there are many clusters of one size, their number
+// at work at once decides, and a cluster of thread blocks has to fit one processing
+// cluster of the GPU: 148, 74, 33, 15, 7 teams of 1, 2, 4, 8, 16 CTAs at once, 15 of
+// nine too, but 7 of eleven.  A CTA per 384 slots, against it (ms, 4th order, equal
+// clusters): 74 of 4096 206 / 113, 148 of 1024 15.8 / 11.9, 296 of 400 5.9 / 4.5,
+// 37 of 4096 at 6th order 43.5 / 26.3 (eight CTAs: 119, 27.4 at 4096).  Few clusters end
+// sooner with it (32 of 256 ... 4096 22.6 / 24.6, eight CTAs 26.0; one of 512 1.30 /
+// 2.11); the team engine asked for by name, which does not weigh engines against one
+// another, takes it.
 constexpr int kEnsTeamSlots = 384, kEnsAutoSlots = 512;
 
 int ens_team_size(int engine, int n)
@@ -741,7 +743,13 @@ int build_groups(hb_ens *e)
     for (int c = 0; c < e->nclusters; ++c) {
         const int n = e->cl[c].n, nch = (n + 31) / 32;
         int C = e->team_ctas;
-        if (C == 0) C = ens_team_size(e->engine, n);
+        if (C == 0) {
+            C = ens_team_size(e->engine, n);
+            // where the device runs as many teams of nine at once
+            if (e->engine != HB_ENGINE_TEAM && C == 8 && cfg_for(8) && cfg_for(9) &&
+                cfg_for(9)->max_teams >= cfg_for(8)->max_teams)
+                C = 9;
+        }
         for (;;) {
             const TeamConfig *cf = cfg_for(C);
             // the automatic choice takes only clusters whose records fit in

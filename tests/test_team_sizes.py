@@ -1,5 +1,5 @@
 """Team sizes chosen by the library.  Ensembles: powers of two of at most 512 slots
-per CTA, which fill the GPU where many clusters are of one size (a CTA per 384
+per CTA, nine in place of eight, which fill the GPU where many clusters are of one size (a CTA per 384
 slots took up to 1.8 times as long there), and the same results as teams of that
 size asked for."""
 import numpy as np
@@ -15,7 +15,7 @@ def test_automatic_sizes():
     sizes = [1, 512, 513, 1024, 1025, 2048, 2049, 4096, 4097, 8000]
     with Ensemble(4, sizes, "fp64") as e:
         assert [e.cluster_engine(c) for c in range(len(sizes))] == \
-            [("team", k) for k in (1, 1, 2, 2, 4, 4, 8, 8, 16, 16)]
+            [("team", k) for k in (1, 1, 2, 2, 4, 4, 9, 9, 16, 16)]
 
 
 def test_same_as_asked_for():
